@@ -140,53 +140,60 @@ static uint64_t stage_key(const Stage& S) {
   return x;
 }
 
-// largest useful split for tile size T: at least one K chunk per K group of the kernel
-static int max_splits(const Stage& S, int T) {
-  int max_chunks = 0;
+// most K chunks of a block: a share keeps at least one
+static int max_chunks(const Stage& S) {
+  int most = 0;
   for (const OutBlock& o : S.outs) {
     int ch = 0;
-    for (int t = o.t0; t < o.t1; ++t) ch += (S.terms[t].k + 15) / 16;
-    max_chunks = std::max(max_chunks, ch);
+    for (int t = o.t0; t < o.t1; ++t) ch += num_chunks(S.terms[t].k);
+    most = std::max(most, ch);
   }
-  return std::max(1, std::min(8, max_chunks / (T == 16 ? 4 : 2)));
+  return most;
 }
+
+static int max_splits(const Stage& S) { return std::max(1, std::min(8, max_chunks(S))); }
 
 // (re)build the stage's tiles for shape (T, splits) and upload them.  Split-K in proportion to
 // the work: the tile with the most K chunks is split over `splits` CTAs, every other tile over
-// ceil(splits x its chunks / the most chunks), each share keeping at least one chunk per K group
-// of the kernel, so that the CTAs of a launch carry about equal work; the CTA entries are ordered
-// by decreasing work.
+// ceil(splits x its chunks / the most chunks), so that the CTAs of a launch carry about equal
+// work; the CTA entries are ordered by decreasing work.
 static int install_stage(Stage& S, int T, int splits) {
   cudaFree(S.d_tiles); cudaFree(S.d_ws); cudaFree(S.d_cnt);
   S.d_tiles = nullptr; S.d_ws = nullptr; S.d_cnt = nullptr;
   finalize_tiles(S, T, T);
   S.splits = splits;
-  const int ks = T == 16 ? 4 : 2;  // K groups of the kernel for this tile size
   const size_t ntiles = S.tiles.size();
-  std::vector<int> ch(ntiles, 0);
   int cmax = 1;
-  for (size_t i = 0; i < ntiles; ++i) {
-    for (int t = S.tiles[i].t0; t < S.tiles[i].t1; ++t) ch[i] += (S.terms[t].k + 15) / 16;
-    cmax = std::max(cmax, ch[i]);
-  }
+  for (const Tile& t : S.tiles) cmax = std::max(cmax, t.nch);
   std::vector<Tile> units;
   int nws = 0;
   for (size_t i = 0; i < ntiles; ++i) {
-    Tile t = S.tiles[i];
-    int np = splits > 1 ? (int)(((int64_t)ch[i] * splits + cmax - 1) / cmax) : 1;
-    np = std::max(1, std::min(np, ch[i] / ks));
-    t.nparts = np;
-    t.cnt_idx = (int)i;
-    t.ws_unit = np > 1 ? nws : 0;
+    const Tile tile = S.tiles[i];
+    int np = splits > 1 ? (int)(((int64_t)tile.nch * splits + cmax - 1) / cmax) : 1;
+    np = std::max(1, std::min(np, tile.nch));
+    const int ws_unit = np > 1 ? nws : 0;
     if (np > 1) nws += np;
+    int term = tile.t0, chunk = 0;  // first chunk of the next share
     for (int q = 0; q < np; ++q) {
+      Tile t = tile;
+      t.nparts = np;
+      t.cnt_idx = (int)i;
+      t.ws_unit = ws_unit;
       t.part = q;
+      t.nch = (int)((int64_t)tile.nch * (q + 1) / np - (int64_t)tile.nch * q / np);
+      t.t0 = term;
+      t.c0 = chunk;
+      for (int c = 0; c < t.nch;) {
+        const int left = num_chunks(S.terms[term].k) - chunk;
+        if (left <= t.nch - c) { c += left; ++term; chunk = 0; }
+        else { chunk += t.nch - c; c = t.nch; }
+      }
       units.push_back(t);
     }
   }
-  std::stable_sort(units.begin(), units.end(), [&](const Tile& a, const Tile& b) {
-    return (int64_t)ch[a.cnt_idx] * b.nparts > (int64_t)ch[b.cnt_idx] * a.nparts;
-  });
+  // work of a unit: its chunks, and the tile's matrix instructions per chunk
+  auto work = [](const Tile& t) { return (int64_t)t.nch * ((t.mt + 15) / 16) * ((t.nt + 7) / 8); };
+  std::stable_sort(units.begin(), units.end(), [&](const Tile& a, const Tile& b) { return work(a) > work(b); });
   S.tiles = std::move(units);
   if (!S.tiles.empty()) {
     CK(cudaMalloc(&S.d_tiles, S.tiles.size() * sizeof(Tile)));
@@ -200,35 +207,31 @@ static int install_stage(Stage& S, int T, int splits) {
   return IMPS_OK;
 }
 
+// Launch shape by estimate.  Tile edge 16 where 32 x 32 tiles would give fewer than one K chunk per
+// SM (a transfer-matrix stage at XXZ D = 512: 9.1 us with 16, 10.3 with 32; with more chunks the
+// fourfold splitting of the operands costs more than it spreads: H_AC at XXZ D = 512 18.5 us with 32,
+// 22.5 with 16, at Hubbard D = 1024 45 and 66).  Shares of as many chunks as leave about three CTAs
+// per SM: H_AC at XXZ D = 512 28.7 us unsplit, 17.8 to 18.7 with 3 to 8 shares; at Hubbard D = 1024
+// 56 unsplit, 49 with 2 or 4, 53 with 8.
+static void shape_estimate(const Stage& S, int* T, int* splits) {
+  constexpr int kSMs = 152;
+  int64_t units = 0;
+  for (const OutBlock& o : S.outs) {
+    if (o.M <= 0 || o.N <= 0) continue;
+    int64_t ch = 0;
+    for (int t = o.t0; t < o.t1; ++t) ch += num_chunks(S.terms[t].k);
+    units += (int64_t)((o.M + 31) / 32) * ((o.N + 31) / 32) * ch;
+  }
+  *T = units < kSMs ? 16 : 32;
+  if (*T == 16) units *= 4;
+  const int64_t per = std::max<int64_t>(1, (units + 3 * kSMs - 1) / (3 * kSMs)), most = max_chunks(S);
+  *splits = (int)std::max<int64_t>(1, std::min<int64_t>(max_splits(S), (most + per - 1) / per));
+}
+
 int upload_stage(Stage& S) {
-  // tile size and split-K: minimise the estimated makespan of the FP64-pipe-bound kernel, the
-  // larger of the heaviest tile's share (a tile's K chunks split over `splits` CTAs) and the
-  // total padded work spread over the 152 SMs
-  constexpr int kSMs = 152, kMaxSplits = 8;
-  auto plan_for = [&](int T, int* splits_out) {
-    int64_t crit = 0, total = 0;
-    int max_chunks = 0;
-    for (const OutBlock& o : S.outs) {
-      int64_t k = 0;
-      int ch = 0;
-      for (int t = o.t0; t < o.t1; ++t) {
-        k += S.terms[t].k;
-        ch += (S.terms[t].k + 15) / 16;
-      }
-      crit = std::max(crit, (int64_t)std::min(T, o.M) * std::min(T, o.N) * k);
-      total += (int64_t)((o.M + T - 1) / T * T) * ((o.N + T - 1) / T * T) * k;
-      max_chunks = std::max(max_chunks, ch);
-    }
-    const int64_t spread = std::max<int64_t>(total / kSMs, 1);
-    int sp = (int)std::min<int64_t>((crit + spread - 1) / spread, kMaxSplits);
-    sp = std::max(1, std::min(sp, max_chunks / (T == 16 ? 4 : 2)));  // at least one chunk per K group
-    *splits_out = sp;
-    return std::max(crit / sp, spread);
-  };
-  int s16 = 1, s32 = 1;
-  const int64_t m16 = plan_for(16, &s16), m32 = plan_for(32, &s32);
-  int T = m16 <= m32 ? 16 : 32;
-  int sp = T == 16 ? s16 : s32;
+  // tile edge and split-K by an estimate; a tuned shape takes its place
+  int T = 32, sp = 1;
+  shape_estimate(S, &T, &sp);
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(stage_key(S));
@@ -283,7 +286,7 @@ int run_stages(imps_plan* p, std::vector<Stage>& stages) {
     if (tc) {
       RC(tc_run_stage(p->tc, S, sl, p->ctx->stream));
     } else {
-      RC(imps_launch_grouped_f64(S.d_tiles, (int)S.tiles.size(), S.d_terms, sl, S.tile_m, S.splits, S.d_ws,
+      RC(imps_launch_grouped_f64(S.d_tiles, (int)S.tiles.size(), S.d_terms, sl, S.tile_m, S.ksteps, S.splits, S.d_ws,
                                  S.d_cnt, p->ctx->stream));
     }
   }
@@ -374,6 +377,7 @@ int imps_ctx_create(int device, imps_ctx** out) {
   int n = 0;
   if (cudaGetDeviceCount(&n) != cudaSuccess || n <= device || device < 0) return IMPS_ERR_NO_DEVICE;
   CK(cudaSetDevice(device));
+  RC(imps_f64_setup());
   imps_ctx* c = new (std::nothrow) imps_ctx();
   if (!c) return IMPS_ERR_OOM;
   c->device = device;
@@ -881,11 +885,11 @@ int imps_plan_autotune(imps_plan* p, int reps, int* n_tuned) {
     if (!have) {
       best.us = std::numeric_limits<float>::infinity();
       for (int T : {16, 32}) {
-        const int smax = max_splits(S, T);
+        const int smax = max_splits(S);
         for (int sp = 1; sp <= smax && !rc; sp *= 2) {
           if ((rc = install_stage(S, T, sp))) break;
           auto launch = [&]() {
-            return imps_launch_grouped_f64(S.d_tiles, (int)S.tiles.size(), S.d_terms, sl, S.tile_m, S.splits,
+            return imps_launch_grouped_f64(S.d_tiles, (int)S.tiles.size(), S.d_terms, sl, S.tile_m, S.ksteps, S.splits,
                                            S.d_ws, S.d_cnt, st);
           };
           if ((rc = launch())) break;  // warm-up

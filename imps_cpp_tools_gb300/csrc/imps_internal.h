@@ -53,7 +53,8 @@ struct Term {
   int32_t k;
   int16_t a_slot, b_slot;
   int8_t a_t, b_t;
-  int8_t pad[6];
+  int16_t kc;      // K chunk length of the term (chunk_len(k))
+  int8_t pad[4];
   double alpha;
 };
 static_assert(sizeof(Term) == 48, "Term layout");
@@ -67,11 +68,25 @@ struct Tile {
   int16_t c_slot;
   int16_t accumulate;  // 1: C += sum, 0: C = sum
   // split-K: the CTA of this entry takes share `part` of `nparts` equal shares of the tile's K
-  // chunks; with nparts > 1 it stores its partial tile at workspace tile ws_unit + part, and the
+  // chunks (t0, c0 and nch below are the share's); with nparts > 1 it stores its partial tile at workspace tile ws_unit + part, and the
   // ticket counter cnt_idx picks the CTA that sums the tile's partials
   int32_t part, nparts, ws_unit, cnt_idx;
+  // the share's first chunk (chunk c0 of term t0) and its number of chunks
+  int32_t c0, nch;
 };
-static_assert(sizeof(Tile) == 56, "Tile layout");
+static_assert(sizeof(Tile) == 64, "Tile layout");
+
+// K chunks of a term: the fewest chunks of at most 16 * kMaxKSteps, of equal length in multiples of
+// 16.  Digit products sum exactly up to K = 113 (kernels_f64.cu); H_AC applies with chunks of at most
+// 96, 80, 64 and 48 took 49.6, 45.3, 45.6 and 49.6 us (Hubbard D = 1024) and 18.5, 18.5, 18.5 and
+// 19.5 us (XXZ D = 512): longer ones cost shared memory for digits, shorter ones more FP64 work.
+constexpr int kMaxKSteps = 5;
+inline int chunk_len(int k) {
+  const int n = k > 0 ? (k + 16 * kMaxKSteps - 1) / (16 * kMaxKSteps) : 1;
+  const int c = (k + n - 1) / n;
+  return c > 0 ? (c + 15) / 16 * 16 : 16;
+}
+inline int num_chunks(int k) { return k > 0 ? (k + chunk_len(k) - 1) / chunk_len(k) : 0; }
 
 // Logical output block with its terms (kept on the host for table export and for the
 // tensor-core packer).
@@ -92,6 +107,7 @@ struct Stage {
   void* d_terms = nullptr;
   int64_t flops = 0;  // useful flops: sum over terms of 2*M*N*K
   int tile_m = 32, tile_n = 32;
+  int ksteps = 1;     // K steps (of 16) of the longest chunk
   // split-K over CTAs (FP64 engine): `splits` CTAs per tile write partial tiles to d_ws and the
   // last one to finish (ticket in d_cnt, reset by it) sums them in a fixed order
   int splits = 1;
@@ -157,6 +173,8 @@ void finalize_tiles(Stage& S, int tm, int tn);
 // ----- kernel launchers (kernels_f64.cu) -----
 struct imps_dslots { double* p[imps::kMaxSlots]; };
 // ntiles: table entries, one CTA each; splits: the largest share count of a tile (> 1 needs the
-// workspace ws and the ticket counters cnt)
-int imps_launch_grouped_f64(const void* d_tiles, int ntiles, const void* d_terms, imps_dslots slots,
-                            int tile_m, int splits, double* ws, int* cnt, void* stream);
+// workspace ws and the ticket counters cnt); tile: 16 or 32; ksteps: K steps of the longest chunk.
+// imps_f64_setup: once per device, before the first launch there
+int imps_f64_setup();
+int imps_launch_grouped_f64(const void* d_tiles, int ntiles, const void* d_terms, imps_dslots slots, int tile,
+                            int ksteps, int splits, double* ws, int* cnt, void* stream);

@@ -1,15 +1,45 @@
-// FP64 kernels for the block-sparse hot path on sm_103a.
+// FP64 grouped GEMM of the block-sparse hot path on sm_103a, on the tensor cores.
 //
-//  * grouped_gemm_f64: output-stationary grouped GEMM over the planner's tile/term tables, one
-//    CTA per table entry: an output tile, or one of `nparts` shares of its K chunks (split-K,
-//    over all of its terms in order; the share count is set per tile by the host); inside a CTA
-//    the chunks are dealt to K groups whose partial tiles are summed in a fixed order.  With one
-//    share the tile is written directly; otherwise every CTA stores its partial tile and the
-//    last CTA of the tile to finish (an atomic ticket after a memory fence; nobody waits) sums
-//    the partials in share order and writes the tile.  Deterministic for a given plan; no
-//    separate zero-fill: the first write also performs the reference's memset of `out`,
-//    VUMPS_helpers.hpp:69.
-//  * Krylov BLAS-1 (reductions without atomics: fixed-grid partials + one finishing block).
+// GB300 retires about 2 FP64 multiply-adds per clock per SM, in its FP64 tensor instruction too (and
+// as few with half the lanes off), but 1035 FP16 ones through mma.sync (all measured); every
+// contraction here was bound by the FP64 pipe.  The kernel therefore splits FP64 operands into exact
+// FP16 digits (the error-free splitting of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59 (2012)
+// 95, in the fixed-point form used on tensor cores by Mukunoki, Ozaki, Ogita and Imamura, ISC 2020):
+//   * a row of op(A), or a column of op(B), inside one K chunk of one term is scaled by a power of
+//     two to magnitude < 1 and rounded to 56 fractional bits (its largest entries keep all 53 bits
+//     of theirs), then written as 7 balanced base-256 digits d_0..d_6, |d_0| <= 256, |d_i| <= 128;
+//   * digit products of one level l = i + j <= 6 (28 of the 49 pairs) are summed in FP32 by mma.sync
+//     m16n8k16.  Every partial sum is an integer of at most 9 * 2^14 * 80 < 2^24, so the sums are
+//     exact in any order; the dropped levels and the rounding of the operands are below 2^-54 of the
+//     product of the two scales;
+//   * per output and chunk the seven level sums are combined in integers, converted to FP64 and added
+//     by one fma: one FP64 instruction where the direct form needs one per k.
+// Relative error of the H_AC apply (2-norm, against a double-double reference): 1.0e-16 to 1.3e-16 over
+// XXZ D = 32 to 1024 and Hubbard D = 64 to 1024, where the direct form had 1.5e-16 (D = 32) to 5.3e-16
+// (XXZ D = 1024); at XXZ D = 512 1.1e-16 after 4.2e-16, at Hubbard D = 1024 1.2e-16 after 4.7e-16.
+// A chunk with an entry that is not finite, or with a row or column whose largest magnitude is outside
+// 2^-423 .. 2^477 (where the scaled sums could leave the FP64 range), is computed by plain FP64
+// fused multiply-adds, so infinities, NaN and extreme scales keep their FP64 results; so is one whose
+// op(A) has at most one entry per row, or op(B) per column (copies by an identity stay exact).
+//
+// mma.sync rather than tcgen05: the operands are split in registers on the fly (no operand packs that
+// could go stale, no extra pass over memory), blocks are ragged with edges from 1 to 82, and the seven
+// level sums of a 16 x 8 sub-tile fit a warp's registers, where a 128-row instruction would compute
+// mostly padding.  What bounds it (XXZ D = 512 H_AC, ncu): integer pipe 29%, tensor pipe 16%, FP64 pipe
+// 13% busy, i.e. the latency of the chain load - split - multiply - combine of one to three chunks per
+// CTA; throughput alone would take about 5 us.
+//
+// Work split: a table entry is an output tile (<= 32 x 32, or <= 16 x 16 where a stage has too few
+// tiles; edges are multiples of 16 and 8, balanced over the block, so that a 68 x 68 block computes
+// 80 x 72 instead of 96 x 96) and a contiguous share of its K chunks.  With one share the tile is
+// written directly; otherwise every CTA stores its partial tile and the last CTA of the tile to
+// finish (an atomic ticket after a memory fence; nobody waits) sums the partials in share order and
+// writes the tile.  Deterministic for a given plan; the first write also performs the reference's
+// memset of `out`, VUMPS_helpers.hpp:69.
+//
+// H_AC apply, direct FP64 form -> this one: XXZ D = 64 23.2 -> 8.2 us, XXZ D = 512 59.4 -> 18.4 us,
+// Hubbard D = 1024 163.7 -> 46.9 us; four-stage transfer matrix at XXZ D = 512 73.8 -> 34.5 us.
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -22,168 +52,352 @@ using imps::Tile;
 
 namespace {
 
-constexpr int TK = 16;
+constexpr int NS = 7;     // digits per operand
+constexpr int kLowExp = 600, kHighExp = 1500;  // biased exponents of rows the split form takes
 
-// Named barrier over the NT threads of one K group (ids 1..KS; 0 is __syncthreads).
-__device__ __forceinline__ void group_sync(int id, int nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
 }
 
-// TMxTN tile computed by KS groups of (TM/RM)*(TN/RN) threads, each thread holding RM x RN
-// accumulators.  The tile's K chunks (TK wide, over all of its terms in order) are dealt
-// round-robin to the KS groups, so a tile with few rows still keeps KS times more warps busy;
-// the groups' partial tiles are summed in a fixed order through shared memory (deterministic).
-template <int TM, int TN, int RM, int RN, int KS>
-__global__ void __launch_bounds__((TM / RM) * (TN / RN) * KS)
-grouped_gemm_f64_kernel(const Tile* __restrict__ tiles, const Term* __restrict__ terms,
-                        imps_dslots slots, double* __restrict__ ws, int* __restrict__ cnt) {
-  constexpr int NT = (TM / RM) * (TN / RN);
-  constexpr int TX = TN / RN;  // threads along n
-  constexpr int AS = TK * (TM + 1), BS = TK * (TN + 1);
-  constexpr int STAGE = KS * (AS + BS);
-  constexpr int RED = (KS - 1) * NT * RM * RN;
-  __shared__ double smem[STAGE > RED ? STAGE : RED];
-  __shared__ int last;
-  const Tile tl = tiles[blockIdx.x];
-  const int splits = tl.nparts, part = tl.part;
-  // this CTA's chunk range [c_lo, c_hi) of the tile's chunk sequence
-  int c_lo = 0, c_hi = 1 << 30;
-  if (splits > 1) {
-    int nch = 0;
-    for (int t = tl.t0; t < tl.t1; ++t) nch += (terms[t].k + TK - 1) / TK;
-    c_lo = (int)((int64_t)nch * part / splits);
-    c_hi = (int)((int64_t)nch * (part + 1) / splits);
-  }
-  const int g = threadIdx.x / NT;
-  const int tid = threadIdx.x - g * NT;
-  const int tx = tid % TX, ty = tid / TX;
-  double* As = smem + g * (AS + BS);  // [TK][TM + 1]
-  double* Bs = As + AS;               // [TK][TN + 1]
-  double acc[RM][RN];
-#pragma unroll
-  for (int i = 0; i < RM; ++i)
-#pragma unroll
-    for (int j = 0; j < RN; ++j) acc[i][j] = 0.0;
+__device__ __forceinline__ void ldsm2(uint32_t (&r)[2], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr) : "memory");
+}
 
-  int chunk = 0;
-  for (int t = tl.t0; t < tl.t1 && chunk < c_hi; ++t) {
-    const Term tm = terms[t];
-    const int nk = (tm.k + TK - 1) / TK;
-    if (chunk + nk <= c_lo) {  // wholly before this split's range
-      chunk += nk;
-      continue;
+__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// x / 2^(E - 1022) as a fixed-point integer with 56 fractional bits (rounded), plus a bias that makes
+// every base-256 digit non-negative: byte i < 6 holds digit d_{6-i} + 128, the top 16 bits d_0 + 512.
+__device__ __forceinline__ uint64_t fixed_digits(double x, int E) {
+  const uint32_t lo = (uint32_t)__double2loint(x);
+  const int32_t hi = __double2hiint(x);
+  const int e = (int)((2u * (uint32_t)hi) >> 21);
+  // the significand in bits 62..10, with the sign (as ones' complement: one unit in bit 0); an entry
+  // below the normal range is far below the row's scale, as is zero
+  const uint32_t sg = (uint32_t)(hi >> 31);
+  const uint32_t th = __funnelshift_l(lo, ((uint32_t)hi & 0x000fffffu) | 0x00100000u, 10) ^ sg, tl = (lo << 10) ^ sg;
+  const int64_t s = (int64_t)(((uint64_t)th << 32) | tl);
+  const int sh = min(E - e + 6, 63);
+  return (uint64_t)(((s >> sh) + (int64_t)(2 * 0x0200808080808080ull + 1)) >> 1);
+}
+
+// the seven digits of two entries (k, k + 1) as packed FP16: 1024 + u, less 1024 and the bias
+__device__ __forceinline__ void digit_pairs(uint64_t x, uint64_t y, uint32_t (&d)[NS]) {
+  const uint32_t xl = (uint32_t)x, yl = (uint32_t)y, xh = (uint32_t)(x >> 32), yh = (uint32_t)(y >> 32);
+  const uint32_t m = 0x64646464u;
+  const uint32_t p0 = __byte_perm(xl, yl, 0x5140), p1 = __byte_perm(xl, yl, 0x7362), p2 = __byte_perm(xh, yh, 0x5140);
+  d[6] = __byte_perm(p0, m, 0x4140);
+  d[5] = __byte_perm(p0, m, 0x4342);
+  d[4] = __byte_perm(p1, m, 0x4140);
+  d[3] = __byte_perm(p1, m, 0x4342);
+  d[2] = __byte_perm(p2, m, 0x4140);
+  d[1] = __byte_perm(p2, m, 0x4342);
+  d[0] = __byte_perm(xh, yh, 0x7632) | 0x64006400u;
+#pragma unroll
+  for (int i = 0; i < NS; ++i) {
+    const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&d[i]),
+                              __half2half2(__ushort_as_half(i == 0 ? 0x6600 : 0x6480)));  // 1536 or 1152
+    d[i] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+}
+
+// One operand's chunk in the registers of four warps: entry (r, k) of op(A) (rows m) or op(B)^T (rows
+// n) is at r * sr + k * sk (one of the strides is 1).  A thread holds the pairs of k at
+// 2 * (lane / 8 + 4 i) of row 8 w + lane % 8: 64 contiguous bytes per row or column of a warp's load,
+// and digit stores that hit 32 banks.  One mapping for both orders keeps the code short: most CTAs
+// run few chunks, and with two mappings a fifth of the stalls were instruction fetches.
+template <int KI>
+__device__ __forceinline__ void load_operand(double (&v)[4 * KI], const double* __restrict__ p, int sr, int sk, int nrow,
+                                             int len, int w, int lane) {
+  const int r = 8 * w + (lane & 7), k0 = 2 * (lane >> 3);
+  const double* __restrict__ pr = p + (int64_t)r * sr + (int64_t)k0 * sk;
+  const int left = r < nrow ? len - k0 : 0;
+#pragma unroll
+  for (int i = 0; i < 2 * KI; ++i)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) v[2 * i + q] = 8 * i + q < left ? pr[(8 * i + q) * (int64_t)sk] : 0.0;
+}
+
+// what a chunk's operands hold (flags of a chunk; side 0: rows of op(A), side 1: columns of op(B))
+enum : int {
+  kUnsplittable = 1,             // an entry that is not finite, a scale outside the split form's range
+  kOne = 2, kSeveral = 4,        // side 0 has a row with one entry that is not zero, with several
+  kOneB = 8, kSeveralB = 16      // side 1
+};
+
+// digits of the held entries into the planes dg[NS][TILE][RS bytes] and the rows' biased exponents into
+// ex[TILE] (1023 for a row of zeros); returns the row's flags
+template <int KI, int TILE>
+__device__ __forceinline__ int store_digits(const double (&v)[4 * KI], int steps, int* ex, unsigned char* dg, int w,
+                                            int lane) {
+  constexpr int RS = 32 * KI + 16, PL = TILE * RS;
+  uint32_t m = 0, any = 0, sum = 0;  // largest exponent field, all low words, the sum of the exponent fields
+#pragma unroll
+  for (int i = 0; i < 4 * KI; ++i) {
+    const uint32_t e2 = 2u * (uint32_t)__double2hiint(v[i]);
+    m = max(m, e2);
+    sum += e2 >> 21;
+    any |= (uint32_t)__double2loint(v[i]);
+  }
+  any |= m;
+#pragma unroll
+  for (int o = 8; o < 32; o <<= 1) {
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    any |= __shfl_xor_sync(0xffffffffu, any, o);
+  }
+  const int E = any == 0 ? 1023 : (int)(m >> 21), r = 8 * w + (lane & 7);
+  if (lane < 8) ex[r] = E;
+  unsigned char* d = dg + r * RS + 4 * (lane >> 3);
+#pragma unroll
+  for (int i = 0; i < 2 * KI; ++i)
+    if (i < 2 * steps) {
+      uint32_t dp[NS];
+      digit_pairs(fixed_digits(v[2 * i], E), fixed_digits(v[2 * i + 1], E), dp);
+#pragma unroll
+      for (int s = 0; s < NS; ++s) *reinterpret_cast<uint32_t*>(d + 16 * i + s * PL) = dp[s];
     }
-    const double* __restrict__ A = slots.p[tm.a_slot] + tm.a_off;
-    const double* __restrict__ B = slots.p[tm.b_slot] + tm.b_off;
-    const double alpha = tm.alpha;
-    for (int k0 = 0; k0 < tm.k; k0 += TK, ++chunk) {
-      if (chunk < c_lo || chunk >= c_hi || (chunk - c_lo) % KS != g) continue;
-      // A tile: rows m0..m0+TM, cols k0..k0+TK of op(A)
-      for (int e = tid; e < TM * TK; e += NT) {
-        int m, k;
-        if (tm.a_t) { k = e % TK; m = e / TK; } else { m = e % TM; k = e / TM; }
-        const int gm = tl.m0 + m, gk = k0 + k;
-        double v = 0.0;
-        if (m < tl.mt && gk < tm.k)
-          v = tm.a_t ? A[(int64_t)gm * tm.a_ld + gk] : A[gm + (int64_t)gk * tm.a_ld];
-        As[k * (TM + 1) + m] = alpha * v;
-      }
-      for (int e = tid; e < TN * TK; e += NT) {
-        int n, k;
-        if (tm.b_t) { n = e % TN; k = e / TN; } else { k = e % TK; n = e / TK; }
-        const int gn = tl.n0 + n, gk = k0 + k;
-        double v = 0.0;
-        if (n < tl.nt && gk < tm.k)
-          v = tm.b_t ? B[gn + (int64_t)gk * tm.b_ld] : B[gk + (int64_t)gn * tm.b_ld];
-        Bs[k * (TN + 1) + n] = v;
-      }
-      group_sync(g + 1, NT);
-      const int kmax = min(TK, tm.k - k0);
-      for (int k = 0; k < kmax; ++k) {
-        double a[RM], b[RN];
+  return (E < kLowExp || E > kHighExp ? kUnsplittable : 0) | (sum > (m >> 21) ? kSeveral : any != 0 ? kOne : 0);
+}
+
+// the level sums of a warp's m16 x n8 sub-tile over the chunk's K steps (16 x 16 tiles: every other
+// one), combined and added to facc
+template <int KI, int TILE>
+__device__ __forceinline__ void chunk_products(const unsigned char* da, const unsigned char* db, const int* ea,
+                                               const int* eb, int m0, int n0, int ks0, int steps, double alpha, int lane,
+                                               double (&facc)[4]) {
+  constexpr int RS = 32 * KI + 16, PL = TILE * RS;
+  float acc[NS][4];
 #pragma unroll
-        for (int i = 0; i < RM; ++i) a[i] = As[k * (TM + 1) + ty + i * (TM / RM)];
+  for (int l = 0; l < NS; ++l)
 #pragma unroll
-        for (int j = 0; j < RN; ++j) b[j] = Bs[k * (TN + 1) + tx + j * TX];
+    for (int q = 0; q < 4; ++q) acc[l][q] = 0.f;
+  // ldmatrix lane addresses: A rows 0-15 x (k 0-7, 8-15); B rows (n) 0-7 x (k 0-7, 8-15)
+  const uint32_t aa = smem_addr(da) + (m0 + (lane & 15)) * RS + (lane >> 4) * 16;
+  const uint32_t ba = smem_addr(db) + (n0 + (lane & 7)) * RS + ((lane >> 3) & 1) * 16;
+  for (int ks = ks0; ks < steps; ks += TILE == 16 ? 2 : 1) {
+    uint32_t b[NS][2];
 #pragma unroll
-        for (int i = 0; i < RM; ++i)
+    for (int s = 0; s < NS; ++s) ldsm2(b[s], ba + s * PL + ks * 32);
 #pragma unroll
-          for (int j = 0; j < RN; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-      }
-      group_sync(g + 1, NT);
+    for (int i = 0; i < NS; ++i) {
+      uint32_t a[4];
+      ldsm4(a, aa + i * PL + ks * 32);
+#pragma unroll
+      for (int s = 0; s + i < NS; ++s) mma_f16(acc[i + s], a, b[s][0], b[s][1]);
     }
   }
-  if (KS > 1) {
-    __syncthreads();  // every group is done with its staging buffers: reuse them for the sums
-    double* red = smem;
-    if (g > 0) {
+  const int g = lane >> 2, t = lane & 3;
 #pragma unroll
-      for (int i = 0; i < RM; ++i)
+  for (int q = 0; q < 4; ++q) {
+    int L[NS];
 #pragma unroll
-        for (int j = 0; j < RN; ++j) red[(((g - 1) * NT + tid) * RM + i) * RN + j] = acc[i][j];
+    for (int l = 0; l < NS; ++l) L[l] = __float2int_rn(acc[l][q]);
+    // sum of L[l] 2^(-8 l), in units of 2^-40: 63 bits and a sign; the lowest 8 bits are rounded off
+    const int64_t hi = ((int64_t)L[0] << 24) + ((int64_t)L[1] << 16) + ((int64_t)L[2] << 8) + L[3];
+    const int64_t lo = ((int64_t)L[4] << 16) + ((int64_t)L[5] << 8) + L[6];
+    const double v = (double)((hi << 16) + ((lo + 128) >> 8));
+    // times 2^(ea + eb - 2044 - 56), by the exponent field (in range: see kLowExp, kHighExp)
+    const int s = ea[m0 + g + (q & 2 ? 8 : 0)] + eb[n0 + 2 * t + (q & 1)] - 2100;
+    const double w = v == 0.0 ? 0.0 : __hiloint2double(__double2hiint(v) + (s << 20), __double2loint(v));
+    facc[q] = fma(alpha, w, facc[q]);
+  }
+}
+
+template <int KI, int TILE>
+__global__ void __launch_bounds__(TILE * 8, TILE == 32 ? 2 : 4)
+grouped_gemm_f64_kernel(const Tile* __restrict__ tiles, const Term* __restrict__ terms,
+                        const __grid_constant__ imps_dslots slots, double* __restrict__ ws,
+                        int* __restrict__ cnt) {
+  constexpr int RS = 32 * KI + 16, PL = TILE * RS;
+  constexpr int NW = TILE / 8;  // warps per operand
+  extern __shared__ __align__(16) unsigned char digits[];
+  __shared__ int ex[2 * TILE];
+  __shared__ int flags[2];  // of an even and an odd chunk
+  __shared__ int last;
+  if (threadIdx.x == 0) flags[0] = flags[1] = 0;
+  __syncthreads();
+  const Tile tl = tiles[blockIdx.x];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // one half of the warps splits op(A), the other op(B), eight rows each (rows past the tile's edge
+  // are left as they are: they reach no output that is written); then each warp takes one 16 x 8
+  // sub-tile, in a 16 x 16 tile with every other K step
+  const int side = warp / NW, w4 = warp % NW;
+  const bool tall = tl.mt > 16;
+  const int m0 = TILE == 32 && tall ? (warp & 1) * 16 : 0;
+  const int n0 = TILE == 16 ? (warp & 1) * 8 : (tall ? warp >> 1 : warp) * 8;
+  const int ks0 = TILE == 16 ? warp >> 1 : 0;
+  const bool mine = n0 < tl.nt, splits = 8 * w4 < (side ? tl.nt : tl.mt);
+  double facc[4] = {0.0, 0.0, 0.0, 0.0};
+
+  struct Chunk {
+    const double *a, *b;
+    int asr, ask, bsr, bsk, len;  // strides along the rows (m, n) and along k
+    double alpha;
+  } cur{}, prev{};
+  double v[4 * KI];
+  bool direct = false;  // the split chunk is to be computed by plain FP64
+  int t = tl.t0, c = tl.c0;
+  // iteration it: load chunk it, multiply chunk it - 1 under the loads, split chunk it
+  for (int it = 0;; ++it) {
+    if (it < tl.nch) {
+      Term tm = terms[t];
+      while (c * tm.kc >= tm.k) {  // this term is done
+        c = 0;
+        tm = terms[++t];
+      }
+      const int k0 = c * tm.kc;
+      ++c;
+      cur.len = min((int)tm.kc, tm.k - k0);
+      cur.alpha = tm.alpha;
+      cur.asr = tm.a_t ? tm.a_ld : 1;
+      cur.ask = tm.a_t ? 1 : tm.a_ld;
+      cur.bsr = tm.b_t ? 1 : tm.b_ld;
+      cur.bsk = tm.b_t ? tm.b_ld : 1;
+      cur.a = slots.p[tm.a_slot] + tm.a_off + (int64_t)tl.m0 * cur.asr + (int64_t)k0 * cur.ask;
+      cur.b = slots.p[tm.b_slot] + tm.b_off + (int64_t)tl.n0 * cur.bsr + (int64_t)k0 * cur.bsk;
+      if (splits)
+        load_operand<KI>(v, side ? cur.b : cur.a, side ? cur.bsr : cur.asr, side ? cur.bsk : cur.ask,
+                         side ? tl.nt : tl.mt, cur.len, w4, lane);
+    }
+    if (it > 0) {
+      const int steps = (prev.len + 15) >> 4;
+      if (mine && !direct) {
+        if (ks0 < steps)
+          chunk_products<KI, TILE>(digits, digits + NS * PL, ex, ex + TILE, m0, n0, ks0, steps, prev.alpha, lane, facc);
+      } else if (mine && ks0 == 0) {
+        // plain FP64; rows and columns past the tile's edge repeat its last ones and are not written
+        const double* a[2];
+        const double* b[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          a[h] = prev.a + (int64_t)min(m0 + (lane >> 2) + 8 * h, tl.mt - 1) * prev.asr;
+          b[h] = prev.b + (int64_t)min(n0 + 2 * (lane & 3) + h, tl.nt - 1) * prev.bsr;
+        }
+#pragma unroll 2
+        for (int k = 0; k < prev.len; ++k) {
+          const double x[2] = {prev.alpha * a[0][(int64_t)k * prev.ask], prev.alpha * a[1][(int64_t)k * prev.ask]};
+          const double y[2] = {b[0][(int64_t)k * prev.bsk], b[1][(int64_t)k * prev.bsk]};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) facc[q] = fma(x[q >> 1], y[q & 1], facc[q]);
+        }
+      }
+      if (it == tl.nch) break;
+      __syncthreads();  // the previous chunk's digits are no longer read
+    } else if (tl.nch == 0) {
+      break;
+    }
+    if (splits) {
+      const int f = store_digits<KI, TILE>(v, (cur.len + 15) >> 4, ex + TILE * side, digits + side * NS * PL, w4, lane);
+      const int fs = (f & kUnsplittable) | (side ? (f & (kOne | kSeveral)) * (kOneB / kOne) : f & (kOne | kSeveral));
+      if (lane < 8 && 8 * w4 + lane < (side ? tl.nt : tl.mt)) atomicOr(&flags[it & 1], fs);
     }
     __syncthreads();
-    if (g > 0) return;  // only group 0 (its own named barrier below) goes on
-    for (int q = 1; q < KS; ++q)
-#pragma unroll
-      for (int i = 0; i < RM; ++i)
-#pragma unroll
-        for (int j = 0; j < RN; ++j) acc[i][j] += red[(((q - 1) * NT + tid) * RM + i) * RN + j];
+    // An operand whose rows (columns) hold one entry each at most selects and scales the other's
+    // entries: plain FP64 gives each its own 53 bits, where the split form would round it to the
+    // scale of its row.
+    const int f = flags[it & 1];
+    direct = (f & kUnsplittable) || (f & (kOne | kSeveral)) == kOne || (f & (kOneB | kSeveralB)) == kOneB;
+    if (threadIdx.x == 0) flags[(it + 1) & 1] = 0;  // written again after the next barrier
+    prev = cur;
   }
-  if (splits > 1) {
-    // partial tile -> workspace; the last CTA of the tile sums all partials in split order
-    double* wp = ws + ((int64_t)tl.ws_unit + part) * (TM * TN);
+  bool writes = mine;
+  if (TILE == 16) {  // the two halves of the K steps
+    __shared__ double half[64 * 4];
+    if (ks0 == 1)
 #pragma unroll
-    for (int i = 0; i < RM; ++i)
+      for (int q = 0; q < 4; ++q) half[q * 64 + threadIdx.x - 64] = facc[q];
+    __syncthreads();
+    writes = mine && ks0 == 0;
+    if (ks0 == 0)
 #pragma unroll
-      for (int j = 0; j < RN; ++j) wp[(ty + i * (TM / RM)) * TN + tx + j * TX] = acc[i][j];
+      for (int q = 0; q < 4; ++q) facc[q] += half[q * 64 + threadIdx.x];
+  }
+
+  if (tl.nparts > 1) {
+    constexpr int WT = TILE * TILE / 4;  // threads that hold outputs
+    // partial tile -> workspace; the last CTA of the tile sums all partials in share order
+    double* wp = ws + ((int64_t)tl.ws_unit + tl.part) * (TILE * TILE) + threadIdx.x;
+    if (writes)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) wp[q * WT] = facc[q];
     __threadfence();
-    group_sync(1, NT);
-    if (tid == 0) last = atomicAdd(cnt + tl.cnt_idx, 1) == splits - 1;
-    group_sync(1, NT);
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(cnt + tl.cnt_idx, 1) == tl.nparts - 1;
+    __syncthreads();
     if (!last) return;
     __threadfence();
+    const double* wr = ws + (int64_t)tl.ws_unit * (TILE * TILE) + threadIdx.x;
+    if (writes) {
 #pragma unroll
-    for (int i = 0; i < RM; ++i)
+      for (int q = 0; q < 4; ++q) facc[q] = 0.0;
+#pragma unroll 4
+      for (int p = 0; p < tl.nparts; ++p)
 #pragma unroll
-      for (int j = 0; j < RN; ++j) {
-        const int e = (ty + i * (TM / RM)) * TN + tx + j * TX;
-        double sum = 0.0;
-        for (int q = 0; q < splits; ++q) sum += __ldcg(ws + ((int64_t)tl.ws_unit + q) * (TM * TN) + e);
-        acc[i][j] = sum;
-      }
-    if (tid == 0) cnt[tl.cnt_idx] = 0;  // re-armed for the next launch of this stage
+        for (int q = 0; q < 4; ++q) facc[q] += __ldcg(wr + p * (TILE * TILE) + q * WT);
+    }
+    if (threadIdx.x == 0) cnt[tl.cnt_idx] = 0;  // re-armed for the next launch of this stage
   }
+  if (!writes) return;
   double* __restrict__ C = slots.p[tl.c_slot] + tl.c_off;
 #pragma unroll
-  for (int i = 0; i < RM; ++i) {
-    const int m = ty + i * (TM / RM);
-    if (m >= tl.mt) continue;
-#pragma unroll
-    for (int j = 0; j < RN; ++j) {
-      const int n = tx + j * TX;
-      if (n >= tl.nt) continue;
-      double* p = C + (tl.m0 + m) + (int64_t)(tl.n0 + n) * tl.c_ld;
-      *p = tl.accumulate ? *p + acc[i][j] : acc[i][j];
-    }
+  for (int q = 0; q < 4; ++q) {
+    const int m = m0 + (lane >> 2) + (q & 2 ? 8 : 0), n = n0 + 2 * (lane & 3) + (q & 1);
+    if (m >= tl.mt || n >= tl.nt) continue;
+    double* p = C + (tl.m0 + m) + (int64_t)(tl.n0 + n) * tl.c_ld;
+    *p = tl.accumulate ? *p + facc[q] : facc[q];
   }
+}
+
+template <int TILE>
+constexpr int smem_bytes(int ki) { return 2 * NS * TILE * (32 * ki + 16); }
+
+using KernelFn = void (*)(const Tile*, const Term*, imps_dslots, double*, int*);
+template <int TILE>
+KernelFn kernel_of(int ki) {
+  switch (ki) {
+    case 1: return grouped_gemm_f64_kernel<1, TILE>;
+    case 2: return grouped_gemm_f64_kernel<2, TILE>;
+    case 3: return grouped_gemm_f64_kernel<3, TILE>;
+    case 4: return grouped_gemm_f64_kernel<4, TILE>;
+    case 5: return grouped_gemm_f64_kernel<5, TILE>;
+    default: return nullptr;
+  }
+}
+
+template <int TILE>
+int setup() {
+  for (int ki = 1; ki <= imps::kMaxKSteps; ++ki)
+    if (cudaFuncSetAttribute((const void*)kernel_of<TILE>(ki), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             smem_bytes<TILE>(ki)) != cudaSuccess)
+      return IMPS_ERR_CUDA;
+  return IMPS_OK;
 }
 
 }  // namespace
 
-int imps_launch_grouped_f64(const void* d_tiles, int ntiles, const void* d_terms, imps_dslots slots,
-                            int tile_m, int splits, double* ws, int* cnt, void* stream) {
+int imps_f64_setup() {
+  const int rc = setup<16>();
+  return rc ? rc : setup<32>();
+}
+
+int imps_launch_grouped_f64(const void* d_tiles, int ntiles, const void* d_terms, imps_dslots slots, int tile,
+                            int ksteps, int splits, double* ws, int* cnt, void* stream) {
   if (ntiles <= 0) return IMPS_OK;
-  if (splits < 1 || (splits > 1 && (!ws || !cnt))) return IMPS_ERR_BAD_ARG;
-  cudaStream_t st = (cudaStream_t)stream;
-  const int grid = ntiles;  // one CTA per table entry (a tile or one K share of it)
+  if (splits < 1 || (splits > 1 && (!ws || !cnt)) || (tile != 16 && tile != 32)) return IMPS_ERR_BAD_ARG;
+  KernelFn fn = tile == 16 ? kernel_of<16>(ksteps) : kernel_of<32>(ksteps);
+  if (!fn) return IMPS_ERR_BAD_ARG;
   imps::count_launch();
-  if (tile_m == 16) {
-    grouped_gemm_f64_kernel<16, 16, 2, 2, 4><<<grid, 256, 0, st>>>((const Tile*)d_tiles, (const Term*)d_terms,
-                                                                  slots, ws, cnt);
-  } else {
-    grouped_gemm_f64_kernel<32, 32, 2, 4, 2><<<grid, 256, 0, st>>>((const Tile*)d_tiles, (const Term*)d_terms,
-                                                                   slots, ws, cnt);
-  }
+  fn<<<ntiles, tile * 8, tile == 16 ? smem_bytes<16>(ksteps) : smem_bytes<32>(ksteps), (cudaStream_t)stream>>>(
+      (const Tile*)d_tiles, (const Term*)d_terms, slots, ws, cnt);
   return cudaGetLastError() == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
 }

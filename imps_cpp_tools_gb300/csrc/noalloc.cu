@@ -21,6 +21,7 @@
 // a loop over one set of layouts copies them once.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 
@@ -52,6 +53,7 @@ static bool ready[kMaxDevices];
 
 struct StageOut {
   int ntiles = 0, nterms = 0;
+  int ksteps = 1;  // K steps of the longest chunk
   bool overflow = false;
 };
 
@@ -88,7 +90,13 @@ bool square_blocks(const imps::Layout& L) {
 }
 
 // emit an output block's tiles (all sharing the block's term range [t0, t1))
-void emit_tiles(StageOut& so, imps::Tile* tiles, int c_slot, int64_t c_off, int ld, int M, int N, int t0, int t1) {
+void emit_tiles(StageOut& so, imps::Tile* tiles, const imps::Term* terms, int c_slot, int64_t c_off, int ld, int M,
+                int N, int t0, int t1) {
+  int chunks = 0;
+  for (int t = t0; t < t1 && t < kNoAllocMaxTerms; ++t) {
+    chunks += imps::num_chunks(terms[t].k);
+    so.ksteps = std::max(so.ksteps, terms[t].kc / 16);
+  }
   for (int n0 = 0; n0 < N; n0 += kTile)
     for (int m0 = 0; m0 < M; m0 += kTile) {
       if (so.ntiles >= kNoAllocMaxTiles) { so.overflow = true; return; }
@@ -107,6 +115,8 @@ void emit_tiles(StageOut& so, imps::Tile* tiles, int c_slot, int64_t c_off, int 
       t.nparts = 1;
       t.ws_unit = 0;
       t.cnt_idx = 0;
+      t.c0 = 0;
+      t.nch = chunks;
     }
 }
 
@@ -118,6 +128,7 @@ void push_term(StageOut& so, imps::Term* terms, int a_slot, int64_t a_off, int a
   t.a_slot = (int16_t)a_slot; t.a_off = a_off; t.a_ld = a_ld > 0 ? a_ld : 1; t.a_t = (int8_t)a_t;
   t.b_slot = (int16_t)b_slot; t.b_off = b_off; t.b_ld = b_ld > 0 ? b_ld : 1; t.b_t = (int8_t)b_t;
   t.k = k;
+  t.kc = (int16_t)imps::chunk_len(k);
   t.alpha = 1.0;
 }
 
@@ -155,6 +166,7 @@ extern "C" int imps_tm_apply_noalloc(const imps_layout* A, const imps_layout* in
       return IMPS_ERR_CUDA;
     }
     d_tables[dev] = (unsigned char*)p;
+    if (imps_f64_setup() != IMPS_OK) return IMPS_ERR_CUDA;
     ready[dev] = true;
   }
   // slots: 0 X (in), 1 Y (out), 2 A, 3 W (static scratch, A's layout)
@@ -171,7 +183,7 @@ extern "C" int imps_tm_apply_noalloc(const imps_layout* A, const imps_layout* in
       if (dir == 0) push_term(s1, h_img.terms[0], SX, X.off, m, 0, SA, b.off, b.rows, 0, b.rows);
       else push_term(s1, h_img.terms[0], SA, b.off, b.rows, 0, SX, X.off, m, 0, b.cols);
     }
-    emit_tiles(s1, h_img.tiles[0], SW, b.off, b.rows, b.rows, b.cols, t0, s1.nterms);
+    emit_tiles(s1, h_img.tiles[0], h_img.terms[0], SW, b.off, b.rows, b.rows, b.cols, t0, s1.nterms);
   }
   // stage 2: Y(q) = sum_b A_b^T W_b (left, Qout(b) = q) or W_b A_b^T (right, Qin(b) = q)
   for (const imps::Block& o : LO.blocks) {
@@ -189,7 +201,7 @@ extern "C" int imps_tm_apply_noalloc(const imps_layout* A, const imps_layout* in
         push_term(s2, h_img.terms[1], SW, b.off, b.rows, 0, SA, b.off, b.rows, 1, b.cols);
       }
     }
-    emit_tiles(s2, h_img.tiles[1], SY, o.off, o.rows, o.rows, o.cols, t0, s2.nterms);
+    emit_tiles(s2, h_img.tiles[1], h_img.terms[1], SY, o.off, o.rows, o.rows, o.cols, t0, s2.nterms);
   }
   if (s1.overflow || s2.overflow) {
     fprintf(stderr, "imps_tm_apply_noalloc: more than %d tiles or %d terms per stage\n", kNoAllocMaxTiles,
@@ -218,7 +230,9 @@ extern "C" int imps_tm_apply_noalloc(const imps_layout* A, const imps_layout* in
   sl.p[SY] = dY;
   sl.p[SA] = const_cast<double*>(dA);
   sl.p[SW] = d_scratch[dev];
-  int rc = imps_launch_grouped_f64(dimg->tiles[0], s1.ntiles, dimg->terms[0], sl, kTile, 1, nullptr, nullptr, stream);
+  int rc = imps_launch_grouped_f64(dimg->tiles[0], s1.ntiles, dimg->terms[0], sl, kTile, s1.ksteps, 1, nullptr, nullptr,
+                                   stream);
   if (rc) return rc;
-  return imps_launch_grouped_f64(dimg->tiles[1], s2.ntiles, dimg->terms[1], sl, kTile, 1, nullptr, nullptr, stream);
+  return imps_launch_grouped_f64(dimg->tiles[1], s2.ntiles, dimg->terms[1], sl, kTile, s2.ksteps, 1, nullptr, nullptr,
+                                 stream);
 }

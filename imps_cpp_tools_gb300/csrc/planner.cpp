@@ -133,25 +133,49 @@ bool square(const Block& B, int m) { return B.rows == m && B.cols == m; }
 
 }  // namespace
 
+// Edges of the tiles of a block edge of length n: the fewest tiles of at most `most`, balanced in
+// multiples of `unit` (the matrix instruction's edge), so that a ragged block pads less.
+static std::vector<int> tile_edges(int n, int most, int unit) {
+  std::vector<int> e;
+  const int units = (n + unit - 1) / unit, per = most / unit, tiles = (units + per - 1) / per;
+  int pos = 0;
+  for (int i = 0; i < tiles; ++i) {
+    e.push_back(pos);
+    pos = std::min(n, pos + unit * (units / tiles + (i < units % tiles ? 1 : 0)));
+  }
+  e.push_back(n);
+  return e;
+}
+
 void finalize_tiles(Stage& S, int tm, int tn) {
   S.tiles.clear();
   S.tile_m = tm;
   S.tile_n = tn;
+  S.ksteps = 1;
+  for (Term& t : S.terms) {
+    t.kc = (int16_t)chunk_len(t.k);
+    S.ksteps = std::max(S.ksteps, t.kc / 16);
+  }
   for (const OutBlock& o : S.outs) {
-    for (int n0 = 0; n0 < o.N; n0 += tn)
-      for (int m0 = 0; m0 < o.M; m0 += tm) {
+    if (o.M <= 0 || o.N <= 0) continue;
+    const std::vector<int> em = tile_edges(o.M, tm, 16), en = tile_edges(o.N, tn, 8);
+    int chunks = 0;
+    for (int t = o.t0; t < o.t1; ++t) chunks += num_chunks(S.terms[t].k);
+    for (size_t j = 0; j + 1 < en.size(); ++j)
+      for (size_t i = 0; i + 1 < em.size(); ++i) {
         Tile t{};
         t.c_off = o.c_off;
         t.c_ld = std::max(o.c_ld, 1);
-        t.m0 = m0;
-        t.n0 = n0;
-        t.mt = std::min(tm, o.M - m0);
-        t.nt = std::min(tn, o.N - n0);
+        t.m0 = em[i];
+        t.n0 = en[j];
+        t.mt = em[i + 1] - em[i];
+        t.nt = en[j + 1] - en[j];
         t.t0 = o.t0;
         t.t1 = o.t1;
         t.c_slot = o.c_slot;
         t.accumulate = o.accumulate;
         t.nparts = 1;
+        t.nch = chunks;
         S.tiles.push_back(t);
       }
   }
