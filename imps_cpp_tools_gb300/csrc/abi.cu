@@ -378,6 +378,7 @@ int imps_ctx_create(int device, imps_ctx** out) {
   if (cudaGetDeviceCount(&n) != cudaSuccess || n <= device || device < 0) return IMPS_ERR_NO_DEVICE;
   CK(cudaSetDevice(device));
   RC(imps_f64_setup());
+  RC(kr_setup());
   imps_ctx* c = new (std::nothrow) imps_ctx();
   if (!c) return IMPS_ERR_OOM;
   c->device = device;
@@ -390,7 +391,7 @@ int imps_ctx_create(int device, imps_ctx** out) {
   CK(cudaMemset(c->dscal, 0, 64 * sizeof(double)));
   CK(cudaMalloc(&c->dflag, 16 * sizeof(int)));
   CK(cudaMemset(c->dflag, 0, 16 * sizeof(int)));
-  c->ws.sync = c->ws.counter + 1;  // counter[0]: last-block reductions; [1], [2]: grid barrier
+  c->ws.sync = c->ws.counter + 1;  // counter[0]: last-block reductions
   c->ws.err = c->dflag + 4;
   CK(cudaMallocHost(&c->hpin, kPinDoubles * sizeof(double) + 16 * sizeof(int)));
   CK(cudaMallocHost(&c->hpin_g, kPinDoubles * sizeof(double) + 16 * sizeof(int)));

@@ -15,10 +15,11 @@ constexpr int kGmresKrylov = 80;  // default restart length of the device GMRES
 struct KrylovWs {
   double* partials = nullptr;     // kr_partials_elems() doubles
   unsigned int* counter = nullptr;
-  unsigned int* sync = nullptr;   // 2 zeroed counters of the cooperative CGS2 step (grid barrier)
+  unsigned int* sync = nullptr;   // 2 zeroed counters of the cooperative CGS2 step (grid barrier, exit)
   int* err = nullptr;             // set when a grid-barrier wait times out
 };
 
+int kr_setup();  // once per device, before the first step there
 size_t kr_partials_elems();
 int kr_multidot(const KrylovWs& ws, const double* V, int64_t ldv, int ncols, const double* w,
                 int64_t n, double* h, int mode, double* out_sqrt, cudaStream_t st);

@@ -212,11 +212,19 @@ __global__ void __launch_bounds__(CT) cgs_pass_kernel(const double* __restrict__
 
 // ---- single-launch CGS2 step (cooperative grid, all blocks co-resident) ----------------------
 // Block b owns rows [b*sub, (b+1)*sub) of w (sub <= COOP_SUB), kept in shared memory through the
-// three passes.  Each reduction is one grid barrier: every block writes its per-column partial
-// sums, then every block sums all partials itself in the same fixed order (identical,
-// reproducible results in every block).  Barrier waits are bounded: on timeout *err is set, the
-// remaining work is skipped, and the exit protocol still resets the counters.
+// three passes; the rows of V that the second pass reads for its dot products are still in L1 when the
+// third reads them for the update.  Each reduction (grid_sums) is one or two grid barriers around sums
+// of the blocks' per-column partials in a fixed order: identical, reproducible results in every block.  Barrier waits are bounded: on timeout *err is
+// set, the remaining work is skipped, and the exit protocol still resets the counters.
+// Bound by the FP64 pipe (a warp's FP64 instruction takes 64 cycles of its scheduler whatever its
+// lanes do), so sums over lanes exchange instead of repeat: a warp adds four columns' lane sums with
+// six additions instead of twenty, and the work is laid out so that the four schedulers get equal
+// shares.  Then come the grid barriers (1.35 us each, measured) and the cooperative launch (4.1 us,
+// 2.0 more than a plain one).  Back to back, at 60 columns, before -> now (and the FP64 work alone):
+// Lanczos steps (second pass full) n = 1,712 39.0 -> 22.6 us (0.4), n = 48,066 43.7 -> 31.5 (10.2),
+// n = 150,276 72.2 -> 55.4 (32.0); GMRES steps (both passes full) n = 24,368 53.7 -> 34.1 us (10.4).
 constexpr int COOP_SUB = 2048;
+constexpr int COOP_RED = 1024;  // doubles of block_dots' scratch
 
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned int* p) {
   unsigned v;
@@ -224,22 +232,22 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned int* p) {
   return v;
 }
 
-// arrival counter sync[0] grows by gridDim.x per barrier; target = k * gridDim.x at barrier k
-__device__ bool grid_barrier(unsigned int* sync, unsigned target, int* err, bool ok) {
+// arrival counter *count grows by the number of participants per barrier; target = k times that at
+// the k-th barrier
+__device__ bool block_barrier(unsigned int* count, unsigned target, int* err, bool ok) {
   __shared__ int good;
   __syncthreads();
   if (threadIdx.x == 0) {
     int g = ok ? 1 : 0;
     __threadfence();
-    atomicAdd(sync, 1u);
+    atomicAdd(count, 1u);
     if (g) {
-      for (long long it = 0; ld_acquire_u32(sync) < target; ++it) {
-        if (it > (1ll << 22) || *(volatile int*)err) {
+      for (long long it = 0; ld_acquire_u32(count) < target; ++it) {
+        if (it > (1ll << 22) || ((it & 63) == 63 && *(volatile int*)err)) {
           atomicExch(err, 1);
           g = 0;
           break;
         }
-        __nanosleep(32);
       }
     }
     good = g;
@@ -248,151 +256,241 @@ __device__ bool grid_barrier(unsigned int* sync, unsigned target, int* err, bool
   return good != 0;
 }
 
-// dst[c] = sum_b P[c*G + b] for c < nc (warps over columns, lanes over blocks, L2 loads)
-__device__ void reduce_partials(const double* P, int G, int nc, double* dst) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int c = warp; c < nc; c += nw) {
-    const double* pc = P + (int64_t)c * G;
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-    int b = lane;
-    for (; b + 96 < G; b += 128) {
-      s0 += __ldcg(pc + b);
-      s1 += __ldcg(pc + b + 32);
-      s2 += __ldcg(pc + b + 64);
-      s3 += __ldcg(pc + b + 96);
-    }
-    for (; b < G; b += 32) s0 += __ldcg(pc + b);
-    const double v = warp_sum((s0 + s1) + (s2 + s3));
-    if (lane == 0) dst[c] = v;
-  }
-}
-
-// P[c*G + block] = sum_{t < len} Vb[t + c*ldv] * x[t]  (x in shared memory)
-__device__ void block_dots(const double* __restrict__ Vb, int64_t ldv, int nc, const double* x, int len,
-                           double* P, int G) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int c0 = warp * 4; c0 < nc; c0 += 4 * nw) {
-    const double* v0 = Vb + (int64_t)min(c0, nc - 1) * ldv;
-    const double* v1 = Vb + (int64_t)min(c0 + 1, nc - 1) * ldv;
-    const double* v2 = Vb + (int64_t)min(c0 + 2, nc - 1) * ldv;
-    const double* v3 = Vb + (int64_t)min(c0 + 3, nc - 1) * ldv;
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-#pragma unroll 2
-    for (int t = lane; t < len; t += 32) {
-      const double xt = x[t];
-      a0 = fma(v0[t], xt, a0);
-      a1 = fma(v1[t], xt, a1);
-      a2 = fma(v2[t], xt, a2);
-      a3 = fma(v3[t], xt, a3);
-    }
-    a0 = warp_sum(a0);
-    a1 = warp_sum(a1);
-    a2 = warp_sum(a2);
-    a3 = warp_sum(a3);
-    if (lane == 0) {
-      P[(int64_t)c0 * G + blockIdx.x] = a0;
-      if (c0 + 1 < nc) P[(int64_t)(c0 + 1) * G + blockIdx.x] = a1;
-      if (c0 + 2 < nc) P[(int64_t)(c0 + 2) * G + blockIdx.x] = a2;
-      if (c0 + 3 < nc) P[(int64_t)(c0 + 3) * G + blockIdx.x] = a3;
-    }
-  }
-}
-
-// x[t] -= sum_c Vb[t + c*ldv] * hs[c]
-__device__ void update_rows(const double* __restrict__ Vb, int64_t ldv, int nc, const double* hs, double* x,
-                            int len) {
-  for (int t = threadIdx.x; t < len; t += blockDim.x) {
-    const double* vr = Vb + t;
-    double a[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    int c = 0;
-    for (; c + 8 <= nc; c += 8) {
+// sum_b p[b] for b < G by one warp (every lane); the loads before the additions, which would
+// otherwise wait for one L2 access after the other
+__device__ __forceinline__ double sum_partials(const double* p, int G) {
+  const int lane = threadIdx.x & 31;
+  double s = 0.0;
+  for (int g = lane; g < G; g += 256) {
+    double y[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) a[q] = fma(-vr[(int64_t)(c + q) * ldv], hs[c + q], a[q]);
-    }
-    for (; c < nc; ++c) a[0] = fma(-vr[(int64_t)c * ldv], hs[c], a[0]);
-    x[t] += ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
+    for (int q = 0; q < 8; ++q) y[q] = __ldcg(p + min(g + q * 32, G - 1));
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (g + q * 32 < G) s += y[q];
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+// The sums over all blocks dst[c] = sum_b P[c*G + b], c < nc, in every block, from partials written
+// before this call; `done`: barriers passed so far.  Up to 16 columns every block sums them itself; of
+// more, the blocks sum a column each and a second barrier publishes the sums (61 columns of 152
+// blocks: 5.5k cycles, where summing all of them in every block took 13.7k).
+__device__ bool grid_sums(const double* P, int G, int nc, double* dst, double* H, unsigned int* sync, int& done,
+                          int* err, bool ok) {
+  ok = block_barrier(sync, (unsigned)++done * G, err, ok);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  if (nc <= nw) {
+    if (ok && warp < nc) {
+      const double s = sum_partials(P + (int64_t)warp * G, G);
+      if (lane == 0) dst[warp] = s;
+    }
+  } else {
+    if (ok)
+      for (int c = blockIdx.x + warp * G; c < nc; c += nw * G) {
+        const double s = sum_partials(P + (int64_t)c * G, G);
+        if (lane == 0) __stcg(H + c, s);
+      }
+    ok = block_barrier(sync, (unsigned)++done * G, err, ok);
+    if (ok)
+      for (int c = threadIdx.x; c < nc; c += blockDim.x) dst[c] = __ldcg(H + c);
+  }
+  __syncthreads();
+  return ok;
+}
+
+// sums over the lanes of four values: afterwards lane l holds that of value 2 * (l / 16) + l / 8 % 2
+__device__ __forceinline__ double warp_sum4(double a0, double a1, double a2, double a3, int lane) {
+  const bool h16 = lane & 16, h8 = lane & 8;
+  const double b0 = (h16 ? a2 : a0) + __shfl_xor_sync(0xffffffffu, h16 ? a0 : a2, 16);
+  const double b1 = (h16 ? a3 : a1) + __shfl_xor_sync(0xffffffffu, h16 ? a1 : a3, 16);
+  double v = (h8 ? b1 : b0) + __shfl_xor_sync(0xffffffffu, h8 ? b0 : b1, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// P[c*G + block] = sum_{t < len} Vb[t + c*ldv] * x[t] for c < nc, and for c == nc (if norm) the sum of
+// x[t]^2; x in shared memory.  A warp's task: four columns over every RS-th slice of 32 rows (the norm
+// is a task of its own).  RS is the split with the least FP64 work on the busiest scheduler: few
+// columns split the rows over many warps, many columns take them whole (fewer lane sums).
+__device__ void block_dots(const double* __restrict__ Vb, int64_t ldv, int nc, bool norm, const double* x, int len,
+                           double* P, int G, double* red) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int ncg = (nc + 3) >> 2, slices = (len + 31) >> 5, ldr = 4 * ncg;
+  int ls = 0, best = 1 << 30;
+#pragma unroll
+  for (int l = 0; l <= 4; ++l) {
+    const int cost = ((ncg << l) + 3) / 4 * (4 * ((slices + (1 << l) - 1) >> l) + 6) + l * ((nc << l) + 127) / 128;
+    if (cost < best && (ncg << l) * 4 <= COOP_RED) {
+      best = cost;
+      ls = l;
+    }
+  }
+  const int RS = 1 << ls, tasks = ncg << ls, step = 32 * RS;
+  for (int task = warp; task < tasks; task += nw) {
+    const int rs = task & (RS - 1), c0 = (task >> ls) * 4;
+    // columns past nc - 1 read column nc - 1 and are not written
+    const double* v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = Vb + (int64_t)min(c0 + q, nc - 1) * ldv;
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    int t = rs * 32 + lane;
+    for (; t + step < len; t += 2 * step) {  // eight loads in flight
+      double y[8];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        y[q] = v[q][t];
+        y[4 + q] = v[q][t + step];
+      }
+      const double x0 = x[t], x1 = x[t + step];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) a[q] = fma(y[q], x0, a[q]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) a[q] = fma(y[4 + q], x1, a[q]);
+    }
+    if (t < len) {
+      const double xt = x[t];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) a[q] = fma(v[q][t], xt, a[q]);
+    }
+    __syncwarp();
+    const double s = warp_sum4(a[0], a[1], a[2], a[3], lane);
+    if ((lane & 7) == 0) red[rs * ldr + c0 + (lane >> 4) * 2 + ((lane >> 3) & 1)] = s;
+  }
+  if (norm && warp == tasks % nw) {
+    double s = 0.0;
+    for (int t = lane; t < len; t += 32) s = fma(x[t], x[t], s);
+    s = warp_sum(s);
+    if (lane == 0) P[(int64_t)nc * G + blockIdx.x] = s;
+  }
+  __syncthreads();
+  for (int i0 = 0; i0 < nc << ls; i0 += blockDim.x) {  // RS lanes per column
+    const int i = i0 + threadIdx.x, c = i >> ls;
+    double s = c < nc ? red[(i & (RS - 1)) * ldr + c] : 0.0;
+    for (int o = 1; o < RS; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (c < nc && (i & (RS - 1)) == 0) P[(int64_t)c * G + blockIdx.x] = s;
+  }
+}
+
+// x[t] -= sum_c Vb[t + c*ldv] * hs[c].  Warps: columns w & 3, + 4, .. (every scheduler then has an
+// equal share) of the row slices w >> 2, + 4, ..; upd: 4 x sub doubles
+__device__ void update_rows(const double* __restrict__ Vb, int64_t ldv, int nc, const double* hs, double* x, int len,
+                            double* upd, int sub) {
+  if (nc <= 4) {
+    for (int t = threadIdx.x; t < len; t += blockDim.x) {
+      double a = x[t];
+      for (int c = 0; c < nc; ++c) a = fma(-Vb[t + (int64_t)c * ldv], hs[c], a);
+      x[t] = a;
+    }
+    __syncthreads();
+    return;
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, cs = warp & 3;
+  for (int s = warp >> 2; s * 32 < len; s += 4) {
+    const int t = s * 32 + lane;
+    const double* vr = Vb + min(t, len - 1);
+    double a = 0.0;
+    int c = cs;
+    for (; c + 28 < nc; c += 32) {  // eight loads in flight; one chain: the pipe, not its latency, is the limit
+      double y[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) y[q] = vr[(int64_t)(c + 4 * q) * ldv];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) a = fma(y[q], hs[c + 4 * q], a);
+    }
+#pragma unroll 4
+    for (; c < nc; c += 4) a = fma(vr[(int64_t)c * ldv], hs[c], a);
+    if (t < len) upd[cs * sub + t] = a;
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < len; t += blockDim.x)
+    x[t] -= (upd[t] + upd[sub + t]) + (upd[2 * sub + t] + upd[3 * sub + t]);
+  __syncthreads();
 }
 
 // c_loc: the first pass projects out columns c_loc..nc-1 only (Lanczos: the two columns the
 // three-term recurrence couples w to; 0 = all columns); the second pass is always full.
-__global__ void __launch_bounds__(CT) cgs2_coop_kernel(const double* __restrict__ V, int64_t ldv, int nc,
+__global__ void __launch_bounds__(CT, 1) cgs2_coop_kernel(const double* __restrict__ V, int64_t ldv, int nc,
                                                       double* __restrict__ w, int64_t n, int sub, double* h,
                                                       double* __restrict__ vnext, int* flag,
                                                       double* __restrict__ partials, unsigned int* sync,
                                                       int* err, int c_loc) {
-  __shared__ double wsm[COOP_SUB];
+  extern __shared__ double dyn[];
+  double* xs = dyn;        // own rows: sub
+  double* upd = xs + sub;  // 4 x sub
   __shared__ double h1[imps::kMaxCols];
   __shared__ double h2[imps::kMaxCols + 1];
+  __shared__ double red[COOP_RED];
   __shared__ double sh[32];
-  __shared__ double beta;
+  __shared__ double beta, inv;
+  __shared__ bool pyth;
   const int G = gridDim.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t base = (int64_t)blockIdx.x * sub;
   const int len = (int)max((int64_t)0, min((int64_t)sub, n - base));
   const double* Vb = V + base;
   double* P0 = partials;
   double* P1 = partials + (int64_t)G * imps::kMaxCols;
   double* P2 = P1 + (int64_t)G * imps::kMaxCols;
+  double* H = P2 + G;  // 2 * kMaxCols published sums
   bool ok = true;
-  for (int t = threadIdx.x; t < len; t += blockDim.x) wsm[t] = w[base + t];
+  for (int t = threadIdx.x; t < len; t += blockDim.x) xs[t] = w[base + t];
   for (int c = threadIdx.x; c < c_loc; c += blockDim.x) h1[c] = 0.0;
   __syncthreads();
   // pass 1: h1 = V^T w over columns c_loc..nc-1
   const int nloc = nc - c_loc;
   const double* Vloc = Vb + (int64_t)c_loc * ldv;
-  block_dots(Vloc, ldv, nloc, wsm, len, P0, G);
-  ok = grid_barrier(sync, (unsigned)G, err, ok);
-  if (ok) reduce_partials(P0, G, nloc, h1 + c_loc);
-  __syncthreads();
-  // pass 2: w -= V h1; h2 = V^T w
+  block_dots(Vloc, ldv, nloc, false, xs, len, P0, G, red);
+  int done = 0;
+  ok = grid_sums(P0, G, nloc, h1 + c_loc, H, sync, done, err, ok);
+  // pass 2: w -= V h1; h2 = V^T w, and |w|^2 as column nc
   if (ok) {
-    update_rows(Vloc, ldv, nloc, h1 + c_loc, wsm, len);
-    __syncthreads();
-    block_dots(Vb, ldv, nc, wsm, len, P1, G);
+    update_rows(Vloc, ldv, nloc, h1 + c_loc, xs, len, upd, sub);
+    block_dots(Vb, ldv, nc, true, xs, len, P1, G, red);
   }
-  // |w|^2 before the second update rides along as column nc of the same partials
-  {
-    double n1 = 0.0;
-    if (ok)
-      for (int t = threadIdx.x; t < len; t += blockDim.x) n1 = fma(wsm[t], wsm[t], n1);
-    n1 = block_sum(n1, sh);
-    if (threadIdx.x == 0) P1[(int64_t)nc * G + blockIdx.x] = n1;
-  }
-  ok = grid_barrier(sync, 2u * G, err, ok);
-  if (ok) reduce_partials(P1, G, nc + 1, h2);  // h2[nc] = |w1|^2
-  __syncthreads();
+  ok = grid_sums(P1, G, nc + 1, h2, H + imps::kMaxCols, sync, done, err, ok);  // h2[nc] = |w1|^2
   // pass 3: w -= V h2; beta = |w|.  V orthonormal: |w2|^2 = |w1|^2 - |h2|^2 exactly, and the
   // second-pass coefficients are tiny unless w1 nearly lies in span(V); then (identically in
   // every block, which all hold the same reduced values) the norm is reduced explicitly.
-  __shared__ bool pyth;
-  if (threadIdx.x == 0) {
+  // The last warp, which has the fewest slices of the update, does this meanwhile (an FP64 square
+  // root or division is some 20 dependent FP64 instructions, and would cost as much in every warp).
+  if (warp == (int)(blockDim.x >> 5) - 1) {
     double s2 = 0.0;
-    for (int c = 0; c < nc; ++c) s2 = fma(h2[c], h2[c], s2);
-    pyth = s2 <= 0.1 * h2[nc];
-    if (pyth) beta = sqrt(h2[nc] - s2);
+    for (int c = lane; c < nc; c += 32) s2 = fma(h2[c], h2[c], s2);
+    s2 = warp_sum(s2);
+    if (lane == 0) {
+      pyth = s2 <= 0.1 * h2[nc];
+      if (pyth) {
+        beta = sqrt(h2[nc] - s2);
+        inv = 1.0 / beta;
+      }
+    }
   }
-  __syncthreads();
-  if (ok) update_rows(Vb, ldv, nc, h2, wsm, len);
+  if (ok) update_rows(Vb, ldv, nc, h2, xs, len, upd, sub);
   __syncthreads();
   if (!pyth) {
     double nacc = 0.0;
     if (ok)
-      for (int t = threadIdx.x; t < len; t += blockDim.x) nacc = fma(wsm[t], wsm[t], nacc);
+      for (int t = threadIdx.x; t < len; t += blockDim.x) nacc = fma(xs[t], xs[t], nacc);
     nacc = block_sum(nacc, sh);
     if (threadIdx.x == 0) P2[blockIdx.x] = nacc;
-    ok = grid_barrier(sync, 3u * G, err, ok);
-    if (ok) reduce_partials(P2, G, 1, sh);  // warp 0 writes sh[0]
-    __syncthreads();
-    if (threadIdx.x == 0 && ok) beta = sqrt(sh[0]);
+    ok = grid_sums(P2, G, 1, sh, H, sync, done, err, ok);
+    if (threadIdx.x == 0 && ok) {
+      beta = sqrt(sh[0]);
+      inv = 1.0 / beta;
+    }
   }
   if (ok) {
     __syncthreads();
     const double bt = beta;
     const bool bad = !(fabs(bt) > 1e-300) || !isfinite(bt);
-    const double inv = bad ? 0.0 : 1.0 / bt;
+    const double sc = bad ? 0.0 : inv;
     for (int t = threadIdx.x; t < len; t += blockDim.x) {
-      w[base + t] = wsm[t];
-      vnext[base + t] = wsm[t] * inv;
+      w[base + t] = xs[t];
+      vnext[base + t] = xs[t] * sc;
     }
     if (blockIdx.x == 0) {
       for (int c = threadIdx.x; c < nc; c += blockDim.x) h[c] = h1[c] + h2[c];
@@ -402,15 +500,17 @@ __global__ void __launch_bounds__(CT) cgs2_coop_kernel(const double* __restrict_
       }
     }
   }
-  // exit: the last block out resets both counters (every block has passed every barrier)
+  // exit: the last block out resets the counters (every block has passed every barrier)
+  __shared__ int out;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    if (atomicAdd(sync + 1, 1u) == (unsigned)G - 1) {
-      sync[0] = 0u;
-      sync[1] = 0u;
-      __threadfence();
-    }
+    out = atomicAdd(sync + 1, 1u) == (unsigned)G - 1;
+  }
+  __syncthreads();
+  if (out) {
+    if (threadIdx.x < 2) sync[threadIdx.x] = 0u;
+    __threadfence();
   }
 }
 
@@ -712,19 +812,21 @@ int kr_cgs2_step(const KrylovWs& ws, const double* V, int64_t ldv, int nc, doubl
   int c_loc = (nloc > 0 && nloc < nc) ? nc - nloc : 0;
   // (column nc of the second partials region carries |w|^2, hence nc < kMaxCols)
   if (ws.sync && ws.err && n <= (int64_t)CGRID * COOP_SUB && nc < kMaxCols) {
-    // one cooperative launch: w stays in shared memory, one grid barrier per reduction
-    int64_t gc = (n + 255) / 256;
+    // one cooperative launch: w stays in shared memory, one grid barrier per reduction.  A block per
+    // 64 rows up to one per SM: the FP64 work of a few hundred rows is longer than the barriers.
+    int64_t gc = (n + 63) / 64;
     if (gc > CGRID) gc = CGRID;
     int64_t subc = (n + gc - 1) / gc;
-    subc = ((subc + 31) / 32) * 32;
+    subc = ((subc + 7) / 8) * 8;
     const int gridc = (int)((n + subc - 1) / subc);
     int subi = (int)subc;
+    const size_t smem = (size_t)5 * subi * sizeof(double);
     double* partials = ws.partials;
     unsigned int* sync = ws.sync;
     int* err = ws.err;
     void* args[] = {(void*)&V, (void*)&ldv, (void*)&nc, (void*)&w, (void*)&n, (void*)&subi, (void*)&h,
                     (void*)&vnext, (void*)&flag, (void*)&partials, (void*)&sync, (void*)&err, (void*)&c_loc};
-    if (cudaLaunchCooperativeKernel((const void*)cgs2_coop_kernel, dim3(gridc), dim3(CT), args, 0, st) ==
+    if (cudaLaunchCooperativeKernel((const void*)cgs2_coop_kernel, dim3(gridc), dim3(CT), args, smem, st) ==
         cudaSuccess) {
       imps::count_launch();
       return IMPS_OK;
@@ -871,6 +973,13 @@ int kr_sign_of_first(const double* x, double* s, cudaStream_t st) {
   imps::count_launch();
   sign_first_kernel<<<1, 32, 0, st>>>(x, s);
   return IMPS_OK;
+}
+
+int kr_setup() {
+  return cudaFuncSetAttribute(cgs2_coop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              5 * COOP_SUB * (int)sizeof(double)) == cudaSuccess
+             ? IMPS_OK
+             : IMPS_ERR_CUDA;
 }
 
 size_t kr_partials_elems() {
