@@ -178,3 +178,35 @@ struct imps_dslots { double* p[imps::kMaxSlots]; };
 int imps_f64_setup();
 int imps_launch_grouped_f64(const void* d_tiles, int ntiles, const void* d_terms, imps_dslots slots, int tile,
                             int ksteps, int splits, double* ws, int* cnt, void* stream);
+
+#ifdef __CUDACC__
+// ----- overlapped launches -----
+// launch_overlapped starts a kernel that may be scheduled while its predecessor in the stream still
+// runs (programmatic dependent launch): the kernel reads only its tables and arguments before
+// wait_for_predecessor(), which every one of its threads executes, and which returns when the
+// predecessor has finished and its writes are visible; whatever follows it in the stream thus finds
+// both done.  allow_successor() lets the next overlapped kernel of the stream be scheduled from here on.
+// Back to back, a plain launch costs 2.06 us on this GPU from one kernel to the next.  Overlapping the
+// grouped GEMMs, the trace and the epilogues: H_AC apply XXZ D = 64 8.2 -> 7.0 us, projected transfer
+// matrix Hubbard D = 1024 60.1 -> 50.9 us, GMRES environment solve XXZ D = 512 5.86 -> 5.33 ms.
+namespace imps {
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_successor() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+inline cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                     A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+}  // namespace imps
+#endif

@@ -116,10 +116,10 @@ __device__ __forceinline__ void digit_pairs(uint64_t x, uint64_t y, uint32_t (&d
 // and digit stores that hit 32 banks.  One mapping for both orders keeps the code short: most CTAs
 // run few chunks, and with two mappings a fifth of the stalls were instruction fetches.
 template <int KI>
-__device__ __forceinline__ void load_operand(double (&v)[4 * KI], const double* __restrict__ p, int sr, int sk, int nrow,
-                                             int len, int w, int lane) {
+__device__ __forceinline__ void load_operand(double (&v)[4 * KI], const double* p, int sr, int sk, int nrow, int len,
+                                             int w, int lane) {
   const int r = 8 * w + (lane & 7), k0 = 2 * (lane >> 3);
-  const double* __restrict__ pr = p + (int64_t)r * sr + (int64_t)k0 * sk;
+  const double* pr = p + (int64_t)r * sr + (int64_t)k0 * sk;
   const int left = r < nrow ? len - k0 : 0;
 #pragma unroll
   for (int i = 0; i < 2 * KI; ++i)
@@ -216,14 +216,14 @@ __device__ __forceinline__ void chunk_products(const unsigned char* da, const un
 template <int KI, int TILE>
 __global__ void __launch_bounds__(TILE * 8, TILE == 32 ? 2 : 4)
 grouped_gemm_f64_kernel(const Tile* __restrict__ tiles, const Term* __restrict__ terms,
-                        const __grid_constant__ imps_dslots slots, double* __restrict__ ws,
-                        int* __restrict__ cnt) {
+                        const __grid_constant__ imps_dslots slots, double* ws, int* cnt) {
   constexpr int RS = 32 * KI + 16, PL = TILE * RS;
   constexpr int NW = TILE / 8;  // warps per operand
   extern __shared__ __align__(16) unsigned char digits[];
   __shared__ int ex[2 * TILE];
   __shared__ int flags[2];  // of an even and an odd chunk
   __shared__ int last;
+  imps::allow_successor();
   if (threadIdx.x == 0) flags[0] = flags[1] = 0;
   __syncthreads();
   const Tile tl = tiles[blockIdx.x];
@@ -247,6 +247,8 @@ grouped_gemm_f64_kernel(const Tile* __restrict__ tiles, const Term* __restrict__
   double v[4 * KI];
   bool direct = false;  // the split chunk is to be computed by plain FP64
   int t = tl.t0, c = tl.c0;
+  if (tl.nch > 0) asm volatile("prefetch.global.L1 [%0];" ::"l"(terms + t));
+  imps::wait_for_predecessor();  // the tables are the plan's own; operands may be its predecessor's results
   // iteration it: load chunk it, multiply chunk it - 1 under the loads, split chunk it
   for (int it = 0;; ++it) {
     if (it < tl.nch) {
@@ -348,7 +350,7 @@ grouped_gemm_f64_kernel(const Tile* __restrict__ tiles, const Term* __restrict__
     if (threadIdx.x == 0) cnt[tl.cnt_idx] = 0;  // re-armed for the next launch of this stage
   }
   if (!writes) return;
-  double* __restrict__ C = slots.p[tl.c_slot] + tl.c_off;
+  double* C = slots.p[tl.c_slot] + tl.c_off;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const int m = m0 + (lane >> 2) + (q & 2 ? 8 : 0), n = n0 + 2 * (lane & 3) + (q & 1);
@@ -397,7 +399,8 @@ int imps_launch_grouped_f64(const void* d_tiles, int ntiles, const void* d_terms
   KernelFn fn = tile == 16 ? kernel_of<16>(ksteps) : kernel_of<32>(ksteps);
   if (!fn) return IMPS_ERR_BAD_ARG;
   imps::count_launch();
-  fn<<<ntiles, tile * 8, tile == 16 ? smem_bytes<16>(ksteps) : smem_bytes<32>(ksteps), (cudaStream_t)stream>>>(
-      (const Tile*)d_tiles, (const Term*)d_terms, slots, ws, cnt);
-  return cudaGetLastError() == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
+  const cudaError_t e =
+      imps::launch_overlapped(fn, dim3(ntiles), dim3(tile * 8), tile == 16 ? smem_bytes<16>(ksteps) : smem_bytes<32>(ksteps),
+                              (cudaStream_t)stream, (const Tile*)d_tiles, (const Term*)d_terms, slots, ws, cnt);
+  return e == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
 }

@@ -419,6 +419,7 @@ __global__ void __launch_bounds__(CT, 1) cgs2_coop_kernel(const double* __restri
                                                       double* __restrict__ partials, unsigned int* sync,
                                                       int* err, int c_loc) {
   extern __shared__ double dyn[];
+  imps::allow_successor();
   double* xs = dyn;        // own rows: sub
   double* upd = xs + sub;  // 4 x sub
   __shared__ double h1[imps::kMaxCols];
@@ -614,9 +615,11 @@ __global__ void axpby_kernel(double a, const double* __restrict__ x, double b, d
 }
 
 // y = x - t + (*s) * rho   (InvEfun_proj epilogue, InvEBlockFunctions.hpp:40-44)
-__global__ void proj_epilogue_kernel(const double* __restrict__ x, const double* __restrict__ t,
-                                     const double* __restrict__ s, const double* __restrict__ rho,
-                                     double* __restrict__ y, int64_t n) {
+__global__ void proj_epilogue_kernel(const double* x, const double* t,
+                                     const double* s, const double* rho,
+                                     double* y, int64_t n) {
+  imps::allow_successor();
+  imps::wait_for_predecessor();
   const double sc = *s;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n;
        r += (int64_t)gridDim.x * blockDim.x)
@@ -631,18 +634,19 @@ __global__ void proj_epilogue_kernel(const double* __restrict__ x, const double*
 // block offsets, cached in shared memory.  Partial sums are combined in a fixed order by the
 // last CTA to finish (gridDim.x <= RB).
 constexpr int kTraceCache = 1024;
-__global__ void __launch_bounds__(RB) trace_prod_kernel(const double* __restrict__ X,
-                                                        const double* __restrict__ R,
+__global__ void __launch_bounds__(RB) trace_prod_kernel(const double* X,
+                                                        const double* R,
                                                         const int64_t* __restrict__ boff,
                                                         const int32_t* __restrict__ bdim,
                                                         const int32_t* __restrict__ bcols, int nb,
-                                                        double* __restrict__ partials,
-                                                        unsigned int* __restrict__ counter,
-                                                        double* __restrict__ out) {
+                                                        double* partials,
+                                                        unsigned int* counter,
+                                                        double* out) {
   __shared__ int64_t so[kTraceCache];
   __shared__ int32_t sm[kTraceCache], sc[kTraceCache];
   __shared__ double sh[32];
   __shared__ bool last;
+  imps::allow_successor();
   const bool cached = nb <= kTraceCache;
   if (cached)
     for (int b = threadIdx.x; b < nb; b += blockDim.x) {
@@ -651,6 +655,7 @@ __global__ void __launch_bounds__(RB) trace_prod_kernel(const double* __restrict
       sc[b] = bcols ? bcols[b] : bdim[b];
     }
   __syncthreads();
+  imps::wait_for_predecessor();  // the block tables are the plan's own
   auto off = [&](int b) -> int64_t { return cached ? so[b] : boff[b]; };
   auto rows = [&](int b) -> int { return cached ? sm[b] : bdim[b]; };
   auto cols = [&](int b) -> int { return cached ? sc[b] : (bcols ? bcols[b] : bdim[b]); };
@@ -896,24 +901,27 @@ int kr_axpby(double a, const double* x, double b, double* y, int64_t n, cudaStre
 int kr_proj_epilogue(const double* x, const double* t, const double* s, const double* rho, double* y,
                      int64_t n, cudaStream_t st) {
   imps::count_launch();
-  proj_epilogue_kernel<<<grid_for(n), 256, 0, st>>>(x, t, s, rho, y, n);
-  return IMPS_OK;
+  const cudaError_t e = imps::launch_overlapped(proj_epilogue_kernel, dim3(grid_for(n)), dim3(256), 0, st, x, t, s, rho, y, n);
+  return e == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
 }
 
 int kr_trace_prod(const KrylovWs& ws, const double* X, const double* R, const int64_t* boff,
                   const int32_t* bdim, int nb, double* out, cudaStream_t st, const int32_t* bcols) {
   imps::count_launch();
   constexpr int grid = 128;  // <= RB: the finishing CTA sums the partials of every CTA
-  trace_prod_kernel<<<grid, RB, 0, st>>>(X, R, boff, bdim, bcols, nb, ws.partials, ws.counter, out);
-  return IMPS_OK;
+  const cudaError_t e = imps::launch_overlapped(trace_prod_kernel, dim3(grid), dim3(RB), 0, st, X, R, boff, bdim, bcols, nb,
+                                                ws.partials, ws.counter, out);
+  return e == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
 }
 
 // out = u - fac * t + tau * rho on split complex planes (fac = c + i s; tau, rho optional):
 //   out_re = u_re - (c t_re - s t_im) + tau_re rho,  out_im = u_im - (s t_re + c t_im) + tau_im rho
-__global__ void fac_epilogue_kernel(const double* __restrict__ ure, const double* __restrict__ uim,
-                                    const double* __restrict__ tre, const double* __restrict__ tim, double c,
-                                    double sn, const double* __restrict__ tau, const double* __restrict__ rho,
-                                    double* __restrict__ ore, double* __restrict__ oim, int64_t n) {
+__global__ void fac_epilogue_kernel(const double* ure, const double* uim,
+                                    const double* tre, const double* tim, double c,
+                                    double sn, const double* tau, const double* rho,
+                                    double* ore, double* oim, int64_t n) {
+  imps::allow_successor();
+  imps::wait_for_predecessor();
   const double tr = tau ? tau[0] : 0.0, ti = tau ? tau[1] : 0.0;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
     const double a = tre[r], b = tim[r];
@@ -927,8 +935,9 @@ int kr_fac_epilogue(const double* ure, const double* uim, const double* tre, con
                     double s, const double* tau, const double* rho, double* ore, double* oim, int64_t n,
                     cudaStream_t st) {
   imps::count_launch();
-  fac_epilogue_kernel<<<grid_for(n), 256, 0, st>>>(ure, uim, tre, tim, c, s, tau, rho, ore, oim, n);
-  return IMPS_OK;
+  const cudaError_t e = imps::launch_overlapped(fac_epilogue_kernel, dim3(grid_for(n)), dim3(256), 0, st, ure, uim, tre,
+                                                tim, c, s, tau, rho, ore, oim, n);
+  return e == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
 }
 
 // Batched form over P systems stacked as [re_0 | im_0 | re_1 | im_1 | ...] (planes of n):
