@@ -379,6 +379,7 @@ int imps_ctx_create(int device, imps_ctx** out) {
   CK(cudaSetDevice(device));
   RC(imps_f64_setup());
   RC(kr_setup());
+  RC(dc_setup());
   imps_ctx* c = new (std::nothrow) imps_ctx();
   if (!c) return IMPS_ERR_OOM;
   c->device = device;
@@ -2372,7 +2373,7 @@ int imps_sector_qr(imps_plan* p, const double* A, double* Q, double* R, int mem)
   if (!D->tall) return IMPS_ERR_UNSUPPORTED;
   cudaStream_t st = p->ctx->stream;
   RC(dc_gather(D->d_ent, (int)D->ent.size(), A, D->dA, st));
-  RC(dc_qr(D->d_mats, (int)D->mats.size(), D->dA, D->dQ, R, D->dir == 1, st));
+  RC(dc_qr(D->mats, D->d_mats, D->dA, D->dQ, R, D->dir == 1, st));
   RC(dc_scatter(D->d_ent, (int)D->ent.size(), D->dQ, Q, st));
   return IMPS_OK;
 }

@@ -59,7 +59,9 @@ int build_decomp(DecompPlan& D, const Layout& A, int dir);
 
 int dc_gather(const GatherEntry* d_ent, int nent, const double* src, double* dense, cudaStream_t st);
 int dc_scatter(const GatherEntry* d_ent, int nent, const double* dense, double* dst, cudaStream_t st);
-int dc_qr(const DenseMat* d_mats, int nmat, double* A, double* Q, double* R, int transpose_r, cudaStream_t st);
+int dc_setup();  // once per device, before the first decomposition there
+int dc_qr(const std::vector<DenseMat>& mats, const DenseMat* d_mats, double* A, double* Q, double* R, int transpose_r,
+          cudaStream_t st);
 // Largest sector dimension N handled by the shared-memory SVD (R and V, N x N each, in shared
 // memory); larger sectors use the global-memory Jacobi kernel.
 constexpr int kJacobiMaxN = 118;
