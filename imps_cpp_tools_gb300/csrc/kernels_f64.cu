@@ -37,8 +37,11 @@
 // writes the tile.  Deterministic for a given plan; the first write also performs the reference's
 // memset of `out`, VUMPS_helpers.hpp:69.
 //
-// H_AC apply, direct FP64 form -> this one: XXZ D = 64 23.2 -> 8.2 us, XXZ D = 512 59.4 -> 18.4 us,
-// Hubbard D = 1024 163.7 -> 46.9 us; four-stage transfer matrix at XXZ D = 512 73.8 -> 34.5 us.
+// H_AC apply, direct FP64 form -> this one: XXZ D = 64 23.2 -> 6.8 us, XXZ D = 512 59.4 -> 16.9 us,
+// Hubbard D = 1024 163.7 -> 42.2 us; four-stage transfer matrix at XXZ D = 512 73.8 -> 32.3 us.
+// Dividing the work between warps that split and warps that multiply, in a persistent CTA per SM, gave
+// 15.5, 38.4 and 29.9 us, but 56.5 for 50.7 us on the projected transfer matrix at Hubbard D = 1024: the
+// SM's issue slots (some 10,000 warp instructions a chunk) are the limit, not the overlap.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -122,9 +125,12 @@ __device__ __forceinline__ void load_operand(double (&v)[4 * KI], const double* 
   const double* pr = p + (int64_t)r * sr + (int64_t)k0 * sk;
   const int left = r < nrow ? len - k0 : 0;
 #pragma unroll
-  for (int i = 0; i < 2 * KI; ++i)
+  for (int s = 0; s < KI; ++s)
+    if (16 * s < len)  // the same for the whole warp; entries of later K steps are not looked at
 #pragma unroll
-    for (int q = 0; q < 2; ++q) v[2 * i + q] = 8 * i + q < left ? pr[(8 * i + q) * (int64_t)sk] : 0.0;
+      for (int i = 2 * s; i < 2 * s + 2; ++i)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) v[2 * i + q] = 8 * i + q < left ? pr[(8 * i + q) * (int64_t)sk] : 0.0;
 }
 
 // what a chunk's operands hold (flags of a chunk; side 0: rows of op(A), side 1: columns of op(B))
@@ -142,12 +148,15 @@ __device__ __forceinline__ int store_digits(const double (&v)[4 * KI], int steps
   constexpr int RS = 32 * KI + 16, PL = TILE * RS;
   uint32_t m = 0, any = 0, sum = 0;  // largest exponent field, all low words, the sum of the exponent fields
 #pragma unroll
-  for (int i = 0; i < 4 * KI; ++i) {
-    const uint32_t e2 = 2u * (uint32_t)__double2hiint(v[i]);
-    m = max(m, e2);
-    sum += e2 >> 21;
-    any |= (uint32_t)__double2loint(v[i]);
-  }
+  for (int s = 0; s < KI; ++s)
+    if (s < steps)
+#pragma unroll
+      for (int i = 4 * s; i < 4 * s + 4; ++i) {
+        const uint32_t e2 = 2u * (uint32_t)__double2hiint(v[i]);
+        m = max(m, e2);
+        sum += e2 >> 21;
+        any |= (uint32_t)__double2loint(v[i]);
+      }
   any |= m;
 #pragma unroll
   for (int o = 8; o < 32; o <<= 1) {
@@ -160,7 +169,7 @@ __device__ __forceinline__ int store_digits(const double (&v)[4 * KI], int steps
   unsigned char* d = dg + r * RS + 4 * (lane >> 3);
 #pragma unroll
   for (int i = 0; i < 2 * KI; ++i)
-    if (i < 2 * steps) {
+    if (i / 2 < steps) {
       uint32_t dp[NS];
       digit_pairs(fixed_digits(v[2 * i], E), fixed_digits(v[2 * i + 1], E), dp);
 #pragma unroll
@@ -332,12 +341,14 @@ grouped_gemm_f64_kernel(const Tile* __restrict__ tiles, const Term* __restrict__
     if (writes)
 #pragma unroll
       for (int q = 0; q < 4; ++q) wp[q * WT] = facc[q];
-    __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(cnt + tl.cnt_idx, 1) == tl.nparts - 1;
+    if (threadIdx.x == 0) {  // the barrier orders the CTA's stores before this thread's fences
+      __threadfence();
+      last = atomicAdd(cnt + tl.cnt_idx, 1) == tl.nparts - 1;
+      __threadfence();
+    }
     __syncthreads();
     if (!last) return;
-    __threadfence();
     const double* wr = ws + (int64_t)tl.ws_unit * (TILE * TILE) + threadIdx.x;
     if (writes) {
 #pragma unroll
