@@ -15,6 +15,10 @@
 //   warps 0-3     : epilogue, tcgen05.ld 32x32b -> FP64 global
 // Every mbarrier wait is bounded; on timeout the CTA records an error, drains what it
 // issued (bounded), frees its TMEM and returns.
+//
+// A tile is latency bound (a few dozen K steps), so two CTAs share an SM, the longest tiles start
+// first, and the kernels' launches overlap.  H_AC apply at Hubbard D = 1024 (209 tiles): 50.1 us with one
+// CTA of four pipeline stages per SM, table order, and the pack kernel's former stores; 28.4 now.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -35,14 +39,14 @@ namespace {
 constexpr int TC_M = 128;        // UMMA M (rows of every tile, zero padded)
 constexpr int TC_NMAX = 128;     // max UMMA N per tile
 constexpr int TC_KSTAGE = 2;     // K-steps (of 16) per pipeline stage
-constexpr int TC_NSTAGE = 4;     // pipeline depth
+constexpr int TC_NSTAGE = 2;     // pipeline depth: two CTAs of two stages per SM, not one of four
 constexpr int TC_THREADS = 128;
 constexpr int A_STAGE_BYTES = TC_KSTAGE * 3 * TC_M * 32;     // 24 KB
 constexpr int B_STAGE_BYTES = TC_KSTAGE * 3 * TC_NMAX * 32;  // 24 KB
 constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
-// the whole opt-in shared memory of the SM: pipeline (4 x 48 KB) + alignment slack + headroom
-// so that every descriptor-addressed access stays inside this CTA's allocation
-constexpr int SMEM_BYTES = 230400;  // 225 KB (opt-in maximum 227 KB minus static shared memory)
+// pipeline (2 x 48 KB) + alignment slack + headroom so that every descriptor-addressed access stays
+// inside this CTA's allocation; two CTAs fit an SM
+constexpr int SMEM_BYTES = 106496;  // 104 KB
 static_assert(TC_NSTAGE * STAGE_BYTES + 1024 <= SMEM_BYTES, "tcgen05 pipeline does not fit");
 constexpr uint32_t WAIT_LIMIT = 1u << 24;
 
@@ -161,48 +165,58 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
 }
 
 // ------------------------------------------------------------------ kernels
-// One block row per job (blockIdx.x), grid-stride over the padded rpad x kpad operand.  The
-// FP64 value is rounded once to FP32 and split there into hi + mid + lo BF16 terms: each
-// difference xf - bf16(xf) is exact in FP32, so the three terms carry all 24 significand bits
-// of xf (relative error 2^-24, the order of the dropped lo*lo-type products) while the FP64
-// pipe, slow on this GPU, sees one conversion per element.  32-bit index arithmetic.
-__global__ void pack_kernel(const PackJob* __restrict__ jobs, imps_dslots slots, __nv_bfloat16* __restrict__ out) {
+// One job per blockIdx.x; its padded rpad x kpad operand in items of eight k of a row, lanes along the
+// rows: an item's BF16 values of one split are the 16 bytes of one core matrix row, so a warp stores
+// 512 contiguous bytes per split.  The FP64 value is rounded once to FP32 and split there into hi + mid
+// + lo BF16 terms: each difference xf - bf16(xf) is exact in FP32, so the three terms carry all 24
+// significand bits of xf (relative error 2^-24, the order of the dropped lo*lo-type products) while the
+// FP64 pipe, slow on this GPU, sees one conversion per element, its bound.  Hubbard D = 1024 H_AC: 17.7
+// us a launch on average with one element per thread, its index divided by rpad and three scattered
+// 2-byte stores; 10.0 now.
+__global__ void __launch_bounds__(256) pack_kernel(const PackJob* __restrict__ jobs, const __grid_constant__ imps_dslots slots,
+                                                   __nv_bfloat16* out) {
+  imps::allow_successor();
   const PackJob jb = jobs[blockIdx.x];
   const double* S = slots.p[jb.slot] + jb.src_off;
-  const int rpad = jb.rpad;
-  const int total = rpad * jb.kpad;
+  const int rpad = jb.rpad, lane = threadIdx.x & 31;
   const float alpha = (float)jb.alpha;
   const int split_elems = rpad * 16;
-  for (int t = threadIdx.x + blockIdx.y * blockDim.x; t < total; t += gridDim.y * blockDim.x) {
-    const int k = t / rpad, r = t - k * rpad;
-    float xf = 0.0f;
-    const int gr = jb.r0 + r;
-    if (r < jb.rows && k < jb.k) {
-      double x;
-      if (jb.role == 0)  // op(A)(gr, k)
-        x = jb.trans ? S[k + (int64_t)gr * jb.src_ld] : S[gr + (int64_t)k * jb.src_ld];
-      else  // op(B)(k, gr)
-        x = jb.trans ? S[gr + (int64_t)k * jb.src_ld] : S[k + (int64_t)gr * jb.src_ld];
-      xf = __double2float_rn(x) * alpha;
+  // entry (row, k) of the operand's row-major form: at row * sr + k * sk
+  const bool kfast = (jb.role == 0) == (jb.trans != 0);
+  const int64_t sr = kfast ? jb.src_ld : 1, sk = kfast ? 1 : jb.src_ld;
+  const int octets = jb.kpad >> 3, wide = (rpad + 31) >> 5;  // items: octet * wide + row group of 32
+  imps::wait_for_predecessor();
+  for (int it = blockIdx.y * 8 + (threadIdx.x >> 5); it < octets * wide; it += gridDim.y * 8) {
+    const int oct = it / wide, r = (it - oct * wide) * 32 + lane;
+    if (r >= rpad) continue;
+    const int k0 = oct * 8;
+    float xf[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      xf[e] = r < jb.rows && k0 + e < jb.k ? __double2float_rn(S[(int64_t)(jb.r0 + r) * sr + (int64_t)(k0 + e) * sk]) * alpha : 0.0f;
+    __nv_bfloat162 w[3][4];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const __nv_bfloat16 hi = __float2bfloat16_rn(xf[e]);
+      const float x1 = xf[e] - __bfloat162float(hi);
+      const __nv_bfloat16 mid = __float2bfloat16_rn(x1);
+      const float x2 = x1 - __bfloat162float(mid);
+      const __nv_bfloat16 lo = __float2bfloat16_rn(x2);
+      __nv_bfloat16* p[3] = {&w[0][e >> 1].x, &w[1][e >> 1].x, &w[2][e >> 1].x};
+      p[0][e & 1] = hi;
+      p[1][e & 1] = mid;
+      p[2][e & 1] = lo;
     }
-    const __nv_bfloat16 hi = __float2bfloat16_rn(xf);
-    const float x1 = xf - __bfloat162float(hi);
-    const __nv_bfloat16 mid = __float2bfloat16_rn(x1);
-    const float x2 = x1 - __bfloat162float(mid);
-    const __nv_bfloat16 lo = __float2bfloat16_rn(x2);
-    const int kstep = k >> 4, kk = k & 15, chunk = kk >> 3, e = kk & 7;
-    const int rgi = r >> 3, rr = r & 7;
-    const int64_t base = jb.dst_off + (int64_t)kstep * 3 * split_elems + (int64_t)chunk * rpad * 8 +
-                         (int64_t)rgi * 64 + rr * 8 + e;
-    out[base] = hi;
-    out[base + split_elems] = mid;
-    out[base + 2 * split_elems] = lo;
+    __nv_bfloat16* d = out + jb.dst_off + (int64_t)(oct >> 1) * 3 * split_elems + (int64_t)(oct & 1) * rpad * 8 + r * 8;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) *reinterpret_cast<uint4*>(d + q * split_elems) = *reinterpret_cast<const uint4*>(w[q]);
   }
 }
 
-__global__ void __launch_bounds__(TC_THREADS, 1)
-tc_gemm_kernel(const TcTile* __restrict__ tiles, const TcTerm* __restrict__ terms,
-               const __nv_bfloat16* __restrict__ packed, imps_dslots slots, int* __restrict__ err) {
+__global__ void __launch_bounds__(TC_THREADS, 2)
+tc_gemm_kernel(const TcTile* __restrict__ tiles, const TcTerm* __restrict__ terms, const __nv_bfloat16* packed,
+               const __grid_constant__ imps_dslots slots, int* err) {
+  imps::allow_successor();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t full_bar[TC_NSTAGE];
@@ -229,6 +243,7 @@ tc_gemm_kernel(const TcTile* __restrict__ tiles, const TcTerm* __restrict__ term
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
+  imps::wait_for_predecessor();  // the packed operands are its predecessor's
   const int nterm = tl.t1 - tl.t0;
   const uint32_t idesc = idesc_bf16(TC_M, tl.npad);
   const uint32_t a_split_bytes = TC_M * 32;          // one split of one K-step (A)
@@ -236,6 +251,7 @@ tc_gemm_kernel(const TcTile* __restrict__ tiles, const TcTerm* __restrict__ term
 
   if (warp == 0 && lane == 0 && nterm > 0) {
     // ---------------- producer
+    asm volatile("fence.proxy.async;" ::: "memory");  // the packs were written through the generic proxy
     int it = 0;
     bool ok = true;
     for (int t = tl.t0; t < tl.t1 && ok; ++t) {
@@ -410,6 +426,13 @@ int tc_create(TcPlan** out, const Plan& P, cudaStream_t st) {
           ts.tiles.push_back(tl);
         }
     }
+    // the tiles with the most matrix instructions first
+    auto work = [&](const TcTile& t) {
+      int64_t k = 0;
+      for (int e = t.t0; e < t.t1; ++e) k += ts.terms[e].ksteps;
+      return k * t.npad;
+    };
+    std::stable_sort(ts.tiles.begin(), ts.tiles.end(), [&](const TcTile& a, const TcTile& b) { return work(a) > work(b); });
     T->stages.push_back(std::move(ts));
   }
   T->packed_elems = off;
@@ -461,10 +484,9 @@ int tc_invalidate(TcPlan* T) {
 
 static int launch_pack(const PackJob* d_jobs, int n, const imps_dslots& slots, __nv_bfloat16* out, cudaStream_t st) {
   if (n <= 0) return IMPS_OK;
-  dim3 grid(n, 4);
   imps::count_launch();
-  pack_kernel<<<grid, 256, 0, st>>>(d_jobs, slots, out);
-  return cudaGetLastError() == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
+  const cudaError_t e = imps::launch_overlapped(pack_kernel, dim3(n, 2), dim3(256), 0, st, d_jobs, slots, out);
+  return e == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
 }
 
 int tc_run_stage(TcPlan* T, const Stage& S, const imps_dslots& slots, cudaStream_t st) {
@@ -481,9 +503,9 @@ int tc_run_stage(TcPlan* T, const Stage& S, const imps_dslots& slots, cudaStream
   if (rc) return rc;
   if (!ts.tiles.empty()) {
     imps::count_launch();
-    tc_gemm_kernel<<<(int)ts.tiles.size(), TC_THREADS, SMEM_BYTES, st>>>(ts.d_tiles, ts.d_terms, T->packed, slots,
-                                                                        T->d_err);
-    if (cudaGetLastError() != cudaSuccess) return IMPS_ERR_CUDA;
+    const cudaError_t e = imps::launch_overlapped(tc_gemm_kernel, dim3((unsigned)ts.tiles.size()), dim3(TC_THREADS),
+                                                  SMEM_BYTES, st, ts.d_tiles, ts.d_terms, T->packed, slots, T->d_err);
+    if (e != cudaSuccess) return IMPS_ERR_CUDA;
   }
   return IMPS_OK;
 }
