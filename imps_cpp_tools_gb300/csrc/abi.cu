@@ -2386,13 +2386,7 @@ int imps_sector_svd(imps_plan* p, const double* A, double* U, double* S, double*
   cudaStream_t st = p->ctx->stream;
   CK(cudaMemsetAsync(D->dstatus, 0, sizeof(int), st));
   RC(dc_gather(D->d_ent, (int)D->ent.size(), A, D->dA, st));
-  int maxN = 0;
-  int64_t maxMN = 0;
-  for (const DenseMat& m : D->mats) {
-    maxN = std::max(maxN, (int)m.N);
-    maxMN = std::max(maxMN, (int64_t)m.M * m.N);
-  }
-  RC(dc_svd(D->d_mats, (int)D->mats.size(), maxN, maxMN, D->dA, S ? S : D->dS, D->dR, D->dW, D->dstatus, st));
+  RC(dc_svd(D->mats, D->d_mats, D->dA, S ? S : D->dS, D->dR, D->dW, D->dstatus, st));
   if (U) RC(dc_scatter(D->d_ent, (int)D->ent.size(), D->dA, U, st));
   if (Viso) {
     if (D->dir == 0) RC(dc_transpose_sq(D->d_mats, (int)D->mats.size(), D->dR, Viso, st));  // V^T
@@ -2413,22 +2407,18 @@ int imps_sector_svd_batch(int np, imps_plan* const* plans, const double* const* 
   cudaStream_t st = c->stream;
   SvdSets sets{};
   sets.nsets = np;
-  int maxN = 0;
-  int64_t maxMN = 0;
+  const std::vector<DenseMat>* mats[kSvdSets] = {};
   for (int k = 0; k < np; ++k) {
     imps_plan* p = plans[k];
     if (!p || p->P.kind != PLAN_DECOMP || p->ctx != c || !A[k] || !p->dc->tall) return IMPS_ERR_BAD_ARG;
     DecompPlan* D = p->dc;
-    for (const DenseMat& m : D->mats) {
-      maxN = std::max(maxN, (int)m.N);
-      maxMN = std::max(maxMN, (int64_t)m.M * m.N);
-    }
+    mats[k] = &D->mats;
     RC(dc_gather(D->d_ent, (int)D->ent.size(), A[k], D->dA, st));
     sets.s[k] = SvdSet{D->d_mats, D->dA, (S && S[k]) ? S[k] : D->dS, D->dR, D->dW, (int)D->mats.size()};
   }
   int* status = plans[0]->dc->dstatus;
   CK(cudaMemsetAsync(status, 0, sizeof(int), st));
-  RC(dc_svd_sets(sets, maxN, maxMN, status, st));
+  RC(dc_svd_sets(sets, mats, status, st));
   for (int k = 0; k < np; ++k) {
     DecompPlan* D = plans[k]->dc;
     if (U && U[k]) RC(dc_scatter(D->d_ent, (int)D->ent.size(), D->dA, U[k], st));

@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(DT) nullspace_kernel(const imps::DenseMat* __r
 }
 
 // One-sided Jacobi SVD of the M x N matrix held in U (in place, M >= N), in global memory (the
-// fallback for N > kJacobiMaxN): on exit U holds the left singular vectors (M x N), S the
+// fallback where neither a cluster's nor one CTA's shared memory holds a sector): on exit U holds the left singular vectors (M x N), S the
 // singular values (descending), V the right singular vectors (N x N).  Round-robin pair
 // ordering; every warp rotates disjoint column pairs.
 __global__ void __launch_bounds__(DT) svd_kernel(const imps::DenseMat* __restrict__ mats,
@@ -551,6 +551,7 @@ __global__ void __launch_bounds__(DT) svd_kernel(const imps::DenseMat* __restric
 }
 
 constexpr int JT = 1024;  // threads of the shared-memory SVD kernels
+constexpr size_t kPjacSmem = 226 * 1024;  // dynamic part; the static flags and sums take < 1 KB
 // every column pair of a round has its own lane group (no loop over pairs in jacobi_sweeps)
 static_assert((imps::kJacobiMaxN + 1) / 2 <= JT / 2, "FP64 sweeps: one 2-lane group per pair");
 static_assert((imps::kMixedMaxN + 1) / 2 <= JT / 16, "FP32 sweeps: one 16-lane group per pair");
@@ -621,8 +622,8 @@ __device__ int jacobi_sweeps(T* B, T* V, int N, int ld, double tol, int max_swee
   return max_sweeps + 1;
 }
 
-// SVD of the M x N sector matrix held in U (M >= N, N <= kJacobiMaxN), with the
-// preconditioning of Drmac and Veselic (SIAM J. Matrix Anal. Appl. 29 (2008) 1322): Householder
+// SVD of the M x N sector matrix held in U (M >= N, N <= kJacobiMaxN) by one CTA, for sectors whose columns
+// do not fit a cluster's shared memory (N = 96: M > 1,470), with the preconditioning of Drmac and Veselic (SIAM J. Matrix Anal. Appl. 29 (2008) 1322): Householder
 // QR with column pivoting A P = Q R, then one-sided Jacobi on the columns of X = R^T, which is
 // strongly graded and converges in a few sweeps (the unpivoted form needs 15-30 sweeps on
 // sectors whose singular values span many decades).  X Vx = Ux S gives R = Vx S Ux^T, so
@@ -765,6 +766,605 @@ __global__ void __launch_bounds__(JT) svd_pjac_kernel(const imps::SvdSets sets, 
   apply_reflectors(a, M, N, tau, u, N);
 }
 
+// ---- sector SVD on a cluster of QC CTAs ---------------------------------------------------------
+// The steps of svd_pjac_kernel (pivoted QR, FP32 then FP64 one-sided Jacobi on the columns of X = R^T) with
+// the work of a sector spread over eight SMs:
+//   * Pivoted QR as in qr_cluster_kernel, columns staying in place: every CTA proposes the longest of its own
+//     remaining columns (its norm summed anew in each update) and the cluster takes the longest of the
+//     eight, so that a step needs one cluster barrier.
+//   * Jacobi by blocks: the columns of B and V are 16 blocks in global memory (L2).  In each of 15 rounds a
+//     CTA loads two blocks, rotates the pairs between them (in the first round also those inside them) in
+//     shared memory, and stores them.  The tangent of a rotation is taken in FP32: it only decides how small
+//     the pair's product becomes.  Cosine and sine are FP64 with c^2 + s^2 = 1 to rounding.
+//   * V of the FP32 sweeps is made orthonormal by two Newton-Schulz steps V <- V (3 - V^T V) / 2 (error
+//     1e-6, 1e-12, rounding); the Cholesky factorisation of the one-CTA form is a serial chain.
+// What bounds it, for a 136 x 68 sector over four decades (one CTA -> cluster, us): the QR, 2,123 -> 345, a
+// chain of two barriers, a remote read, square root and division a step; the FP32 sweeps, 635 -> 433, the
+// latency of a turn (920 cycles: 280 to load and multiply, 210 parameters, 130 to store); the FP64 sweeps,
+// 3,060 -> 458, FP64 instructions at 64 cycles a warp; the products, 300 -> 77; U, 795 -> 157.  The polar
+// step of XXZ D = 512 (both directions, 42 sectors): 6,690 -> 1,547 us.  20 equal sectors of N columns:
+// N = 1 27 -> 27 us, 4 131 -> 81, 16 707 -> 377, 64 5,806 -> 1,259, 118 34,322 -> 4,231, so every sector that
+// fits comes here.
+constexpr int JB = 2 * QC;  // column blocks
+constexpr int SVD_MAXN = 256;
+constexpr int SVD_SMEM = 216 * 1024;
+constexpr int SVD_SMEM2 = 102 * 1024;  // with two CTAs on an SM
+
+// shared memory (doubles) of an M x N sector: the columns of A with two reflectors and two candidates, and
+// then in turn the Jacobi blocks; own columns of two N x N matrices and kc columns of a third; own columns of U
+__host__ __device__ constexpr size_t svd_base_doubles(int M, int N) { return ((size_t)(N + QC - 1) / QC + 4) * M; }
+__host__ __device__ constexpr size_t svd_work_doubles(int M, int N, int kc, bool u_shared) {
+  const size_t own = (N + QC - 1) / QC, bs = (N + JB - 1) / JB;
+  size_t w = 4 * bs * N;
+  const size_t prod = 2 * own * N + (size_t)kc * (N | 1), u = u_shared ? own * M : 0;
+  if (prod > w) w = prod;
+  return u > w ? u : w;
+}
+
+__device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
+  cluster_arrive();
+  cluster_wait();
+}
+__device__ __forceinline__ int ld_cluster(const int* p, uint32_t rank) {
+  uint32_t a = (uint32_t)__cvta_generic_to_shared(p), b;
+  int v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(a), "r"(rank));
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(b) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_cluster(double* p, uint32_t rank, double v) {
+  uint32_t a = (uint32_t)__cvta_generic_to_shared(p), b;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(a), "r"(rank));
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(b), "d"(v) : "memory");
+}
+
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float y;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// tan of the rotation for zeta = (be - al) / (2 ga), to FP32 rounding (0 for zeta beyond 1e19)
+__device__ __forceinline__ float tangent(float zeta) {
+  return __fdividef(copysignf(1.f, zeta), fabsf(zeta) + sqrt_approx(fmaf(zeta, zeta, 1.f)));
+}
+// x 2^-(e - 1023) as a float, truncated; 0 if that is below the normal floats (e: at least x's exponent field)
+__device__ __forceinline__ float scaled_float(double x, int e) {
+  const int hi = __double2hiint(x), ex = ((hi >> 20) & 0x7ff) - e + 127;
+  const int m = (hi & 0xfffff) << 3 | (unsigned)__double2loint(x) >> 29;
+  return ex > 0 ? __int_as_float((hi & 0x80000000) | ex << 23 | m) : 0.f;
+}
+
+// The rotation that makes two columns with squared norms al, be and product ga orthogonal, and the new
+// squared norms; false if |ga| <= tol sqrt(al be) already.  mr, mt: the largest |ga| / sqrt(al be) and
+// |tangent| so far.
+__device__ __forceinline__ bool rotation(float& al, float& be, float ga, float tol, float& c, float& s, float& mr,
+                                         float& mt) {
+  const float ratio = fabsf(ga) * rsqrtf(al) * rsqrtf(be);
+  if (!(ratio > tol)) return false;
+  const float t = tangent(__fdividef(be - al, 2.f * ga));
+  mr = fmaxf(mr, ratio);
+  mt = fmaxf(mt, fabsf(t));
+  c = rsqrtf(fmaf(t, t, 1.f));
+  s = c * t;
+  al = fmaf(-t, ga, al);
+  be = fmaf(t, ga, be);
+  return true;
+}
+__device__ __forceinline__ bool rotation(double& al, double& be, double ga, double tol, double& c, double& s, float& mr,
+                                         float& mt) {
+  const int ea = (__double2hiint(al) >> 20) & 0x7ff, eb = (__double2hiint(be) >> 20) & 0x7ff;
+  const int e = max(ea, eb);
+  double t;
+  if (e - min(ea, eb) < 100 && e > 200 && e < 1900) {
+    const float gf = scaled_float(ga, e), ratio = fabsf(gf) * rsqrtf(scaled_float(al, e) * scaled_float(be, e));
+    if (!(ratio > (float)tol)) return false;
+    mr = fmaxf(mr, ratio);
+    const float zeta = __fdividef(scaled_float(be - al, e), 2.f * gf);
+    t = fabsf(zeta) > 1e9f ? __fdividef(0.5f, zeta) : tangent(zeta);
+  } else {
+    if (!(ga != 0.0 && fabs(ga) > tol * sqrt(al) * sqrt(be))) return false;
+    const double zeta = (be - al) / (2.0 * ga);
+    t = copysign(1.0, zeta) / (fabs(zeta) + sqrt(fma(zeta, zeta, 1.0)));
+    mr = 1.f;
+  }
+  mt = fmaxf(mt, fabsf((float)t));
+  const double u = t * t;
+  if (u < 0x1p-14) {  // (1 + u)^-1/2 by its series; the next term is below 2^-57
+    c = fma(u, fma(u, fma(u, -0.3125, 0.375), -0.5), 1.0);
+  } else {
+    double y = rsqrtf((float)(1.0 + u));
+#pragma unroll
+    for (int i = 0; i < 2; ++i) y = fma(0.5 * y, fma(-(1.0 + u) * y, y, 1.0), y);  // Newton: 2^-22, 2^-43, rounding
+    c = y;
+  }
+  s = c * t;
+  al = fma(-t, ga, al);
+  be = fma(t, ga, be);
+  return true;
+}
+
+// One-sided Jacobi sweeps on the columns of B (N x N, global memory), the rotations into V, until every pair
+// has |<b_i, b_j>| <= tol |b_i| |b_j|: the sweep rotated nothing, or so little that it left no more.  (A pair
+// that the sweep has made orthogonal gets products back from later rotations of either column with a third:
+// at most N of the size mr max(mr, mt), for the largest ratio |<b_i, b_j>| / |b_i| |b_j| and tangent that
+// the sweep met; so `rest` = tol / N does.)  nrm_g: squared column norms (scratch).  An FP64 instruction takes 64 cycles of its
+// scheduler however many lanes it serves and a round of N = 68 has 5 pairs, so a pair has 16 lanes: warps
+// 0-3 take products, parameters and B, the others V, one turn behind.
+// G lanes per pair with R rows each (N <= G R; loops of fixed length: a branch per step cost 20 cycles each).
+// Returns the sweeps run, max_sweeps + 1 if the last one still rotated.
+struct SweepShared {
+  double nrm[2 * SVD_MAXN / JB], rc[2][SVD_MAXN / JB], rs[2][SVD_MAXN / JB];
+  int rij[2][SVD_MAXN / JB];  // rotations of this turn and the one before: columns i, j or -1
+  int flag[2];
+};
+template <typename T, int G, int R>
+__device__ int cluster_sweeps(T* B, T* V, T* nrm_g, int N, T tol, float rest, int max_sweeps, T* sm, SweepShared& sh,
+                              int rank) {
+  constexpr int PAIRS = 128 / G, RV = (R * G + 31) / 32;
+  T* nrm = (T*)sh.nrm;
+  T(*rc)[SVD_MAXN / JB] = (T(*)[SVD_MAXN / JB])sh.rc;
+  T(*rs)[SVD_MAXN / JB] = (T(*)[SVD_MAXN / JB])sh.rs;
+  int(*rij)[SVD_MAXN / JB] = sh.rij;
+  int* flag = sh.flag;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gl = threadIdx.x & (G - 1);
+  const int nblk = min(JB, max(2, N + (N & 1)));  // fewer columns than blocks: a column each
+  auto start = [&](int b) { return b * N / nblk; };
+  for (int sweep = 0; sweep < max_sweeps; ++sweep) {
+    if (threadIdx.x < 2) flag[threadIdx.x] = 0;
+    float mr = 0.f, mt = 0.f;
+    for (int r = 0; r < nblk - 1; ++r) {
+      const int p = rank == 0 ? nblk - 1 : (r + rank) % (nblk - 1);
+      const int q = rank == 0 ? r : (r - rank + QC * (nblk - 1)) % (nblk - 1);
+      const bool on = rank < nblk / 2;  // else no blocks
+      const int sp = start(p), np = on ? start(p + 1) - sp : 0, sq = start(q), nq = on ? start(q + 1) - sq : 0;
+      const int n2 = np + nq;
+      T *b = sm, *v = sm + (size_t)n2 * N;
+      auto global_of = [&](int e) { return e < np * N ? sp * N + e : (sq - np) * N + e; };
+#pragma unroll 4
+      for (int e = threadIdx.x; e < n2 * N; e += QT) {
+        const int g = global_of(e);
+        const T x = __ldcg(B + g), y = __ldcg(V + g);
+        b[e] = x;
+        v[e] = y;
+      }
+      if (r == 0) {
+        __syncthreads();
+        for (int i = warp; i < n2; i += QT / 32) {
+          T a2 = 0;
+          for (int e = lane; e < N; e += 32) a2 = fma(b[(size_t)i * N + e], b[(size_t)i * N + e], a2);
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+          if (lane == 0) nrm[i] = a2;
+        }
+      } else if (threadIdx.x < n2) {
+        nrm[threadIdx.x] = __ldcg(nrm_g + ((int)threadIdx.x < np ? sp + threadIdx.x : sq - np + threadIdx.x));
+      }
+      __syncthreads();
+      // r = 0: all pairs of both blocks, by the circle schedule; else those between the blocks
+      const int P = n2 + (n2 & 1), m = max(np, nq), turns = r == 0 ? P - 1 : m, pairs = r == 0 ? P / 2 : np;
+      const int nb = min(4, (pairs * G + 31) / 32);  // warps with pairs; V: the others, idle schedulers first
+      const int vw = warp < nb ? -1 : (warp & 3) >= nb ? (warp >> 2) * (4 - nb) + (warp & 3) - nb : warp + 4 - 2 * nb;
+      for (int t = 0; t <= turns; ++t) {
+        if (warp < nb && t < turns) {
+          for (int k0 = 0; k0 < pairs; k0 += PAIRS) {
+            const int k = k0 + threadIdx.x / G;
+            int i = 0, j = n2;
+            if (k < pairs) {
+              if (r > 0) {
+                i = k;
+                j = k + t < m ? k + t : k + t - m;
+                j = j < nq ? np + j : n2;
+              } else {
+                i = k == 0 ? t : (t + k) % (P - 1);
+                j = k == 0 ? P - 1 : (t - k + P - 1) % (P - 1);
+                if (i > j) { const int z = i; i = j; j = z; }
+              }
+            }
+            const bool valid = j < n2;
+            if (!valid) j = 0;  // loads without branches: of any column, past the end of the last element
+            T *bp = b + (size_t)i * N, *bq = b + (size_t)j * N;
+            T x[R], y[R], ga = 0, al, be, c = 1, s = 0;
+#pragma unroll
+            for (int u = 0; u < R; ++u) {
+              const int e = min(gl + u * G, N - 1);
+              x[u] = bp[e];
+              y[u] = bq[e];
+            }
+            al = nrm[i];
+            be = nrm[j];
+#pragma unroll
+            for (int u = 0; u < R; ++u) {
+              ga = fma(gl + u * G < N ? x[u] : (T)0, y[u], ga);
+            }
+            if (G == 32) ga += __shfl_xor_sync(0xffffffffu, ga, 16);
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) ga += __shfl_xor_sync(0xffffffffu, ga, o);
+            const bool turn = valid && rotation(al, be, ga, tol, c, s, mr, mt);
+            if (gl == 0 && k < pairs) {
+              rij[t & 1][k] = turn ? i << 16 | j : -1;
+              if (turn) {
+                rc[t & 1][k] = c;
+                rs[t & 1][k] = s;
+                nrm[i] = al;
+                nrm[j] = be;
+              }
+            }
+            if (turn) {
+#pragma unroll
+              for (int u = 0; u < R; ++u) {
+                const int e = gl + u * G;
+                const T xn = c * x[u] - s * y[u], yn = s * x[u] + c * y[u];
+                if (e < N) {
+                  bp[e] = xn;
+                  bq[e] = yn;
+                }
+              }
+            }
+          }
+        }
+        if (vw >= 0 && t > 0) {
+          const int h = (t - 1) & 1;
+          for (int k = vw; k < pairs; k += 8 - nb) {
+            const int ij = rij[h][k];
+            if (ij < 0) continue;
+            T *vp = v + (size_t)(ij >> 16) * N, *vq = v + (size_t)(ij & 0xffff) * N;
+            const T c = rc[h][k], s = rs[h][k];
+            T x[RV], y[RV];
+#pragma unroll
+            for (int u = 0; u < RV; ++u) {
+              const int e = min(lane + u * 32, N - 1);
+              x[u] = vp[e];
+              y[u] = vq[e];
+            }
+#pragma unroll
+            for (int u = 0; u < RV; ++u) {
+              const int e = lane + u * 32;
+              const T xn = c * x[u] - s * y[u], yn = s * x[u] + c * y[u];
+              if (e < N) {
+                vp[e] = xn;
+                vq[e] = yn;
+              }
+            }
+          }
+        }
+        __syncthreads();
+      }
+#pragma unroll 4
+      for (int e = threadIdx.x; e < n2 * N; e += QT) {
+        const int g = global_of(e);
+        __stcg(B + g, b[e]);
+        __stcg(V + g, v[e]);
+      }
+      if (threadIdx.x < n2)
+        __stcg(nrm_g + ((int)threadIdx.x < np ? sp + threadIdx.x : sq - np + threadIdx.x), nrm[threadIdx.x]);
+      if (r == nblk - 2 && gl == 0 && mr > 0.f) {  // non-negative floats compare as integers
+        atomicMax(flag, __float_as_int(mr));
+        atomicMax(flag + 1, __float_as_int(mt));
+      }
+      if (r == nblk - 2) __syncthreads();
+      cluster_sync();
+    }
+    int ir = 0, it = 0;
+    for (int c = 0; c < QC; ++c) {
+      ir = max(ir, ld_cluster(flag, c));
+      it = max(it, ld_cluster(flag + 1, c));
+    }
+    cluster_sync();  // every flag has been read before it is reset
+    mr = __int_as_float(ir);
+    if (mr * fmaxf(mr, __int_as_float(it)) <= rest) return sweep + 1;
+  }
+  return max_sweeps + 1;
+}
+
+// ... for N up to SVD_MAXN
+template <typename T>
+__device__ int cluster_sweeps(T* B, T* V, T* nrm_g, int N, T tol, float rest, int max_sweeps, T* sm, SweepShared& sh,
+                              int rank) {
+#define IMPS_SWEEPS(G, R) return cluster_sweeps<T, G, R>(B, V, nrm_g, N, tol, rest, max_sweeps, sm, sh, rank)
+  switch ((N + 15) / 16) {
+    case 0: case 1: case 2: IMPS_SWEEPS(16, 2);
+    case 3: IMPS_SWEEPS(16, 3);
+    case 4: IMPS_SWEEPS(16, 4);
+    case 5: IMPS_SWEEPS(16, 5);
+    case 6: IMPS_SWEEPS(16, 6);
+    case 7: case 8: IMPS_SWEEPS(16, 8);
+    default: IMPS_SWEEPS(32, 8);
+  }
+#undef IMPS_SWEEPS
+}
+
+__global__ void __cluster_dims__(QC, 1, 1) __launch_bounds__(QT, 2)
+svd_cluster_kernel(const imps::SvdSets sets, int smem_doubles, int max_sweeps, int* __restrict__ status) {
+  extern __shared__ double qsm[];
+  __shared__ double tau_s[SVD_MAXN], beta_s[SVD_MAXN], sig[SVD_MAXN];
+  __shared__ int piv[SVD_MAXN], perm[SVD_MAXN];
+  __shared__ double tail_s[32], cand[2][QC][5];  // candidates of all CTAs: norm^2, column, beta, tau, scale
+  __shared__ int done_s[32];
+  __shared__ SweepShared sweep_s;
+  // the widest sectors first: they get SMs of their own, and the narrow ones fill up
+  int bi = blockIdx.x / QC, ks = 0;
+  const int total = gridDim.x / QC;
+  const auto locate = [&](int g, int& k) {
+    for (k = 0; k + 1 < sets.nsets && g >= sets.s[k].n; ++k) g -= sets.s[k].n;
+    return g;
+  };
+  if (total <= SVD_MAXN) {
+    for (int g = threadIdx.x; g < total; g += QT) {
+      const int l = locate(g, ks);
+      perm[g] = sets.s[ks].mats[l].N;
+    }
+    __syncthreads();
+    for (int g = threadIdx.x; g < total; g += QT) {
+      int rk = 0;
+      for (int h = 0; h < total; ++h) rk += (perm[h] > perm[g] || (perm[h] == perm[g] && h < g)) ? 1 : 0;
+      piv[rk] = g;
+    }
+    __syncthreads();
+    bi = piv[bi];
+    __syncthreads();
+  }
+  bi = locate(bi, ks);
+  const imps::DenseMat mt = sets.s[ks].mats[bi];
+  const int M = mt.M, N = mt.N, rank = (int)cluster_rank();
+  if (N <= 0 || M < N) return;  // the whole cluster
+  double* U = sets.s[ks].U + mt.q_off;
+  double* S = sets.s[ks].S + mt.s_off;
+  double* Vo = sets.s[ks].V + mt.r_off;
+  double* W = sets.s[ks].W + mt.w_off + N;  // M * N doubles of scratch
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = QT / 32;
+  const int own = (N + QC - 1) / QC, mine = N > rank ? (N - rank + QC - 1) / QC : 0;
+  double* cols = qsm;                     // own columns rank + QC * jl of A
+  double* vcand = cols + (size_t)own * M; // 2 x M: this CTA's candidate column
+  double* vbuf = vcand + 2 * (size_t)M;   // 2 x M: the step's reflector
+  double* buf = vbuf + 2 * (size_t)M;
+  const int room = smem_doubles - (int)svd_base_doubles(M, N);
+
+  // ---- A P = Q R
+  for (int jl = warp; jl < mine; jl += nw) {
+    double t = 0.0;
+    for (int i = lane; i < M; i += 32) {
+      const double x = U[i + (int64_t)(rank + QC * jl) * M];
+      cols[(size_t)jl * M + i] = x;
+      if (i > 0) t = fma(x, x, t);
+    }
+    t = wsum(t);
+    if (lane == 0) {
+      tail_s[jl] = t;
+      done_s[jl] = 0;
+    }
+  }
+  cluster_sync();  // every CTA of the cluster has started
+  for (int k = 0; k < N; ++k) {
+    const int par = k & 1;
+    // the longest own column that is left, in every warp; squared norms compare as integers (one that is
+    // not a number counts as 0, so that every step finds a column)
+    double n2 = 0.0;
+    long long key = -1;
+    int bj = lane;
+    if (lane < mine && !done_s[lane]) {
+      const double x = cols[(size_t)lane * M + k];
+      n2 = fma(x, x, tail_s[lane]);
+      key = n2 >= 0.0 ? __double_as_longlong(n2) : 0;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const long long ok = __shfl_xor_sync(0xffffffffu, key, o);
+      const int oj = __shfl_xor_sync(0xffffffffu, bj, o);
+      if (ok > key || (ok == key && oj < bj)) { key = ok; bj = oj; }
+    }
+    if (key >= 0) {
+      const double* c = cols + (size_t)bj * M;
+      for (int i = k + threadIdx.x; i < M; i += QT) vcand[(size_t)par * M + i] = c[i];
+    }
+    if (warp == 0) {
+      double beta = 0.0, tau = 0.0, scal = 0.0;
+      n2 = __shfl_sync(0xffffffffu, n2, bj);
+      if (key >= 0) {
+        const double x0 = cols[(size_t)bj * M + k];
+        beta = x0;
+        if (tail_s[bj] > 0.0) {
+          beta = -copysign(sqrt(n2), x0);
+          // both quotients in one division: tau in even lanes, the scale in odd ones
+          const double q = (lane & 1 ? 1.0 : beta - x0) / (lane & 1 ? x0 - beta : beta);
+          tau = __shfl_sync(0xffffffffu, q, 0);
+          scal = __shfl_sync(0xffffffffu, q, 1);
+        }
+      }
+      if (lane < QC) {
+        double* d = cand[par][rank];
+        st_cluster(d, lane, key >= 0 ? __longlong_as_double(key) : -1.0);
+        st_cluster(d + 1, lane, (double)(rank + QC * bj));
+        st_cluster(d + 2, lane, beta);
+        st_cluster(d + 3, lane, tau);
+        st_cluster(d + 4, lane, scal);
+      }
+    }
+    cluster_sync();
+    int cr = 0, ci = 0;  // the longest of the eight (ties: the smallest index)
+    key = -1;
+    for (int r = 0; r < QC; ++r) {
+      const double cn = cand[par][r][0];
+      const long long ok = __double_as_longlong(cn);
+      const int oi = (int)cand[par][r][1];
+      if (ok >= 0 && (ok > key || (ok == key && oi < ci))) { key = ok; ci = oi; cr = r; }
+    }
+    const double tau = cand[par][cr][3], scal = cand[par][cr][4];
+    double* v = vbuf + (size_t)par * M;
+    for (int i = k + threadIdx.x; i < M; i += QT) {
+      const double x = ld_cluster(vcand + (size_t)par * M + i, cr);
+      v[i] = i == k ? 1.0 : scal * x;
+    }
+    if (threadIdx.x == 0) {
+      piv[k] = ci;
+      tau_s[k] = tau;
+      beta_s[k] = cand[par][cr][2];
+      if (cr == rank) done_s[ci / QC] = 1;
+    }
+    __syncthreads();
+    for (int jl = warp; jl < mine; jl += nw) {
+      double* c = cols + (size_t)jl * M;
+      if (cr == rank && jl == ci / QC) {
+        for (int i = k + lane; i < M; i += 32) c[i] = v[i];
+      } else if (!done_s[jl]) {
+        double w = 0.0, t = 0.0;
+        if (tau != 0.0) {
+          for (int i = k + lane; i < M; i += 32) w = fma(v[i], c[i], w);
+          w = -tau * wsum(w);
+        }
+        for (int i = k + lane; i < M; i += 32) {
+          const double y = tau != 0.0 ? fma(w, v[i], c[i]) : c[i];
+          c[i] = y;
+          if (i > k + 1) t = fma(y, y, t);
+        }
+        t = wsum(t);
+        if (lane == 0) tail_s[jl] = t;
+      }
+    }
+    __syncthreads();
+  }
+
+  // ---- X = R^T (lower triangular) in U's place, its FP32 copy scaled to about 1, and V = 1
+  float* Xf = (float*)Vo;
+  float* Vf = Xf + (size_t)N * N;
+  const int eb = (__double2hiint(beta_s[0]) >> 20) & 0x7ff;
+  const double xs = eb > 0 && eb < 2046 ? __hiloint2double((2046 - eb) << 20, 0) : 1.0;
+  for (int i = warp; i < N; i += nw) {  // column i of R is column piv[i] of A
+    if (piv[i] % QC != rank) continue;
+    const double* c = cols + (size_t)(piv[i] / QC) * M;
+    for (int j = lane; j < N; j += 32) {
+      const double x = j < i ? c[j] : j == i ? beta_s[i] : 0.0;
+      __stcg(U + i + (int64_t)j * N, x);
+      __stcg(Xf + i + (size_t)j * N, (float)(x * xs));
+      __stcg(Vf + i + (size_t)j * N, i == j ? 1.f : 0.f);
+    }
+  }
+  cluster_sync();
+  cluster_sweeps<float>(Xf, Vf, (float*)S, N, 1e-5f, 1e-5f, 8, (float*)buf, sweep_s, rank);
+
+  // ---- V orthonormal in FP64, every CTA its own columns rank + QC * jl (N x own in shared memory)
+  const int ld = N | 1;
+  double* vc = buf;
+  double* yc = vc + (size_t)own * N;
+  double* part = yc + (size_t)own * N;  // kc columns of an N x N matrix
+  const int kc = min(N, (room - 2 * own * N) / ld);
+  // out = a0 out + a1 F in, or out = F^T in; F: N x N in global memory; `held`: it is in `part` already
+  auto product = [&](const double* F, bool trans, const double* in, double* out, double a0, double a1, bool held) {
+    for (int k0 = 0; k0 < N; k0 += kc) {
+      const int nk = min(kc, N - k0);
+      __syncthreads();
+      if (!held || kc < N) {
+        for (int k = warp; k < nk; k += nw)
+          for (int i = lane; i < N; i += 32) part[i + (size_t)k * ld] = __ldcg(F + i + (int64_t)(k0 + k) * N);
+        __syncthreads();
+      }
+      const int nr = trans ? nk : N;
+      for (int e = threadIdx.x; e < nr * mine; e += QT) {
+        const int jl = e / nr, i = e - jl * nr;
+        double a = 0.0;
+        if (trans) {
+          const double *f = part + (size_t)i * ld, *x = in + (size_t)jl * N;
+#pragma unroll 4
+          for (int r = 0; r < N; ++r) a = fma(f[r], x[r], a);
+          out[k0 + i + (size_t)jl * N] = a;
+        } else {
+          const double *f = part + i, *x = in + (size_t)jl * N + k0;
+#pragma unroll 4
+          for (int k = 0; k < nk; ++k) a = fma(f[(size_t)k * ld], x[k], a);
+          double* o = out + i + (size_t)jl * N;
+          *o = fma(a1, a, k0 > 0 ? *o : a0 == 0.0 ? 0.0 : a0 * *o);
+        }
+      }
+    }
+    __syncthreads();
+  };
+  auto publish = [&](double* g, const double* c) {
+    for (int jl = warp; jl < mine; jl += nw)
+      for (int i = lane; i < N; i += 32) __stcg(g + i + (int64_t)(rank + QC * jl) * N, c[i + (size_t)jl * N]);
+    cluster_sync();
+  };
+  for (int jl = warp; jl < mine; jl += nw)
+    for (int i = lane; i < N; i += 32) vc[i + (size_t)jl * N] = (double)__ldcg(Vf + i + (size_t)(rank + QC * jl) * N);
+  __syncthreads();
+  publish(W, vc);
+  for (int pass = 0; pass < 2; ++pass) {
+    const double* F = pass == 0 ? W : Vo;
+    product(F, true, vc, yc, 0.0, 1.0, false);
+    product(F, false, yc, vc, 1.5, -0.5, true);
+    publish(pass == 0 ? Vo : W, vc);
+  }
+  // ---- B = X V in V's place, and the FP64 sweeps
+  product(U, false, vc, yc, 0.0, 1.0, false);
+  publish(Vo, yc);
+  const double tol = (double)N * 2.220446049250313e-16;
+  const int sw = cluster_sweeps<double>(Vo, W, S, N, tol, 2e-16f, max_sweeps, buf, sweep_s, rank);
+  if (threadIdx.x == 0 && rank == 0 && sw > max_sweeps && status) atomicExch(status, 1);
+
+  // ---- singular values, descending (ties by index; what is not a number last), in every CTA
+  for (int j = warp; j < N; j += nw) {
+    double a2 = 0.0;
+    for (int i = lane; i < N; i += 32) {
+      const double x = __ldcg(Vo + i + (int64_t)j * N);
+      a2 = fma(x, x, a2);
+    }
+    a2 = wsum(a2);
+    if (lane == 0) sig[j] = sqrt(a2);
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < N; j += QT) {
+    const double sj = sig[j] >= 0.0 ? sig[j] : -1.0;
+    int rk = 0;
+    for (int i = 0; i < N; ++i) {
+      const double si = sig[i] >= 0.0 ? sig[i] : -1.0;
+      rk += (si > sj || (si == sj && i < j)) ? 1 : 0;
+    }
+    perm[rk] = j;
+  }
+  __syncthreads();
+  // V = P Ux: row piv[i] of V = row i of B / sigma; through shared memory, as B is in V's place
+  for (int jl = warp; jl < mine; jl += nw) {
+    const int pj = perm[rank + QC * jl];
+    const double sj = sig[pj];
+    for (int i = lane; i < N; i += 32) {
+      const double x = __ldcg(Vo + i + (int64_t)pj * N);
+      buf[piv[i] + (size_t)jl * N] = sj > 0.0 ? x / sj : 0.0;
+    }
+  }
+  cluster_sync();
+  for (int jl = warp; jl < mine; jl += nw) {
+    const int j = rank + QC * jl;
+    for (int i = lane; i < N; i += 32) Vo[i + (int64_t)j * N] = buf[i + (size_t)jl * N];
+    if (lane == 0) S[j] = sig[perm[j]];
+  }
+  __syncthreads();
+  // U = Q [Vx; 0], own columns; reflector k - 1 is on its way while k is applied
+  const bool u_shared = own * M <= room;
+  double* uc = u_shared ? buf : U + (int64_t)rank * M;  // column jl at uc + jl * ldu
+  const int64_t ldu = u_shared ? M : (int64_t)QC * M;
+  for (int jl = warp; jl < mine; jl += nw) {
+    const int pj = perm[rank + QC * jl];
+    for (int i = lane; i < M; i += 32) uc[i + jl * ldu] = i < N ? __ldcg(W + i + (int64_t)pj * N) : 0.0;
+  }
+  auto fetch = [&](int k) {
+    const double* src = cols + (size_t)(piv[k] / QC) * M;
+    for (int i = k + threadIdx.x; i < M; i += QT) vbuf[(size_t)(k & 1) * M + i] = ld_cluster(src + i, piv[k] % QC);
+  };
+  fetch(N - 1);
+  __syncthreads();
+  for (int k = N - 1; k >= 0; --k) {
+    if (k > 0) fetch(k - 1);
+    if (tau_s[k] != 0.0)
+      for (int jl = warp; jl < mine; jl += nw) reflect(uc + jl * ldu, vbuf + (size_t)(k & 1) * M, tau_s[k], M, k, lane);
+    __syncthreads();
+  }
+  __syncwarp();
+  cluster_arrive();
+  if (u_shared)
+    for (int jl = warp; jl < mine; jl += nw)
+      for (int i = lane; i < M; i += 32) U[i + (int64_t)(rank + QC * jl) * M] = buf[i + (size_t)jl * M];
+  cluster_wait();  // no CTA leaves while another may still read its columns
+}
+
 // Y = X (M x N) transposed into (N x M), per matrix (used for V^T outputs)
 __global__ void transpose_kernel(const imps::DenseMat* __restrict__ mats, const double* __restrict__ X,
                                  double* __restrict__ Y, int use_r) {
@@ -816,7 +1416,12 @@ int dc_scatter(const GatherEntry* d_ent, int nent, const double* dense, double* 
 }
 
 int dc_setup() {
-  return cudaFuncSetAttribute(qr_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, QR_SMEM) == cudaSuccess
+  const auto smem = [](const void* kernel, size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+  };
+  return smem((const void*)qr_cluster_kernel, QR_SMEM) && smem((const void*)svd_cluster_kernel, SVD_SMEM) &&
+                 smem((const void*)svd_pjac_kernel<false>, kPjacSmem) &&
+                 smem((const void*)svd_pjac_kernel<true>, kPjacSmem)
              ? IMPS_OK
              : IMPS_ERR_CUDA;
 }
@@ -845,19 +1450,39 @@ int dc_nullspace(const DenseMat* d_mats, int nmat, double* A, double* NS, cudaSt
   return cudaGetLastError() == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
 }
 
-int dc_svd(const DenseMat* d_mats, int nmat, int maxN, int64_t maxMN, double* U, double* S, double* V, double* W,
+int dc_svd(const std::vector<DenseMat>& mats, const DenseMat* d_mats, double* U, double* S, double* V, double* W,
            int* status, cudaStream_t st) {
   SvdSets sets{};
   sets.nsets = 1;
-  sets.s[0] = SvdSet{d_mats, U, S, V, W, nmat};
-  return dc_svd_sets(sets, maxN, maxMN, status, st);
+  sets.s[0] = SvdSet{d_mats, U, S, V, W, (int)mats.size()};
+  const std::vector<DenseMat>* m = &mats;
+  return dc_svd_sets(sets, &m, status, st);
 }
 
-int dc_svd_sets(const SvdSets& sets, int maxN, int64_t maxMN, int* status, cudaStream_t st) {
+int dc_svd_sets(const SvdSets& sets, const std::vector<DenseMat>* const* mats, int* status, cudaStream_t st) {
   if (sets.nsets < 1 || sets.nsets > kSvdSets) return IMPS_ERR_BAD_ARG;
-  int nmat = 0;
-  for (int k = 0; k < sets.nsets; ++k) nmat += sets.s[k].n;
+  int nmat = 0, maxN = 0;
+  int64_t maxMN = 0;
+  size_t least = 0, good = 0, want = 0;  // shared memory (doubles) of the cluster kernel
+  for (int k = 0; k < sets.nsets; ++k) {
+    nmat += sets.s[k].n;
+    for (const DenseMat& m : *mats[k]) {
+      maxN = std::max(maxN, (int)m.N);
+      maxMN = std::max(maxMN, (int64_t)m.M * m.N);
+      const size_t base = svd_base_doubles(m.M, m.N);
+      least = std::max(least, base + svd_work_doubles(m.M, m.N, std::min(m.N, 16), false));
+      good = std::max(good, base + svd_work_doubles(m.M, m.N, std::min(m.N, 16), true));
+      want = std::max(want, base + svd_work_doubles(m.M, m.N, m.N, true));
+    }
+  }
   if (nmat <= 0) return IMPS_OK;
+  if (maxN <= SVD_MAXN && least * sizeof(double) <= (size_t)SVD_SMEM) {
+    imps::count_launch();
+    // two CTAs per SM if U still fits, with the products in pieces
+    const size_t doubles = std::min(want, (size_t)(good * sizeof(double) <= SVD_SMEM2 ? SVD_SMEM2 : SVD_SMEM) / sizeof(double));
+    svd_cluster_kernel<<<nmat * QC, QT, doubles * sizeof(double), st>>>(sets, (int)doubles, 30, status);
+    return cudaGetLastError() == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
+  }
   if (maxN > kJacobiMaxN) {  // global-memory fallback, one launch per set
     for (int k = 0; k < sets.nsets; ++k) {
       if (sets.s[k].n <= 0) continue;
@@ -868,22 +1493,12 @@ int dc_svd_sets(const SvdSets& sets, int maxN, int64_t maxMN, int* status, cudaS
     return cudaGetLastError() == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
   }
   imps::count_launch();
-  constexpr size_t kSmemMax = 226 * 1024;  // dynamic part; the static flags and sums take < 1 KB
   const bool mixed = maxN <= kMixedMaxN;
   const int64_t ld = maxN | 1;
   const size_t base = ((size_t)(mixed ? 3 : 2) * ld * maxN + 2 * (size_t)maxN) * 8 + (size_t)2 * maxN * 4 + 16;
-  const int a_smem = base + (size_t)maxMN * 8 <= kSmemMax ? 1 : 0;
+  const int a_smem = base + (size_t)maxMN * 8 <= kPjacSmem ? 1 : 0;
   const size_t bytes = base + (a_smem ? (size_t)maxMN * 8 : 0);
-  if (bytes > kSmemMax) return IMPS_ERR_TOO_LARGE;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(svd_pjac_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(svd_pjac_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax) !=
-            cudaSuccess)
-      return IMPS_ERR_CUDA;
-    attr_set = true;
-  }
+  if (bytes > kPjacSmem) return IMPS_ERR_TOO_LARGE;
   if (mixed) svd_pjac_kernel<true><<<nmat, JT, bytes, st>>>(sets, a_smem, 20, status);
   else svd_pjac_kernel<false><<<nmat, JT, bytes, st>>>(sets, a_smem, 30, status);
   return cudaGetLastError() == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;

@@ -62,12 +62,12 @@ int dc_scatter(const GatherEntry* d_ent, int nent, const double* dense, double* 
 int dc_setup();  // once per device, before the first decomposition there
 int dc_qr(const std::vector<DenseMat>& mats, const DenseMat* d_mats, double* A, double* Q, double* R, int transpose_r,
           cudaStream_t st);
-// Largest sector dimension N handled by the shared-memory SVD (R and V, N x N each, in shared
-// memory); larger sectors use the global-memory Jacobi kernel.
+// Largest sector dimension N of the one-CTA shared-memory SVD (R and V, N x N each, in shared memory), for
+// sectors that do not fit a cluster's; still larger ones use the global-memory Jacobi kernel.
 constexpr int kJacobiMaxN = 118;
 // Largest N of the mixed-precision SVD (R, V and an FP32 / scratch square in shared memory).
 constexpr int kMixedMaxN = 96;
-int dc_svd(const DenseMat* d_mats, int nmat, int maxN, int64_t maxMN, double* U, double* S, double* V, double* W,
+int dc_svd(const std::vector<DenseMat>& mats, const DenseMat* d_mats, double* U, double* S, double* V, double* W,
            int* status, cudaStream_t st);
 // Up to kSvdSets independent sector SVDs (e.g. the two polar steps of a site update) in one
 // launch: set k's sectors are CTAs [sum_{j<k} n_j, sum_{j<=k} n_j).
@@ -81,7 +81,8 @@ struct SvdSets {
   SvdSet s[kSvdSets];
   int nsets;
 };
-int dc_svd_sets(const SvdSets& sets, int maxN, int64_t maxMN, int* status, cudaStream_t st);
+// mats[k]: the sectors of set k on the host
+int dc_svd_sets(const SvdSets& sets, const std::vector<DenseMat>* const* mats, int* status, cudaStream_t st);
 int dc_colscale(const DenseMat* d_mats, int nmat, double* X, const double* S, double power, cudaStream_t st);
 int dc_transpose_sq(const DenseMat* d_mats, int nmat, const double* X, double* Y, cudaStream_t st);
 int dc_nullspace(const DenseMat* d_mats, int nmat, double* A, double* NS, cudaStream_t st);
