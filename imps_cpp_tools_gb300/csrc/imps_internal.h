@@ -113,6 +113,9 @@ struct Stage {
   int splits = 1;
   double* d_ws = nullptr;
   int* d_cnt = nullptr;
+  int planes = 1;  // operand sets that one launch may take: each has its own part of d_ws and d_cnt
+  int64_t ws_len = 0;
+  int cnt_len = 0;
 };
 
 enum SlotKind { SLOT_EXTERNAL = 0, SLOT_INTERNAL = 1 };
@@ -172,11 +175,20 @@ void finalize_tiles(Stage& S, int tm, int tn);
 
 // ----- kernel launchers (kernels_f64.cu) -----
 struct imps_dslots { double* p[imps::kMaxSlots]; };
+// the operand sets of a launch (grid.y), and the length of one's part of the workspace and the counters
+struct imps_planes {
+  imps_dslots s[2];
+  int n;
+  int cnt_len;
+  int64_t ws_len;
+};
 // ntiles: table entries, one CTA each; splits: the largest share count of a tile (> 1 needs the
 // workspace ws and the ticket counters cnt); tile: 16 or 32; ksteps: K steps of the longest chunk.
 // imps_f64_setup: once per device, before the first launch there
 int imps_f64_setup();
 int imps_launch_grouped_f64(const void* d_tiles, int ntiles, const void* d_terms, imps_dslots slots, int tile,
+                            int ksteps, int splits, double* ws, int* cnt, void* stream);
+int imps_launch_grouped_f64(const void* d_tiles, int ntiles, const void* d_terms, const imps_planes& planes, int tile,
                             int ksteps, int splits, double* ws, int* cnt, void* stream);
 
 #ifdef __CUDACC__

@@ -225,7 +225,7 @@ __device__ __forceinline__ void chunk_products(const unsigned char* da, const un
 template <int KI, int TILE>
 __global__ void __launch_bounds__(TILE * 8, TILE == 32 ? 2 : 4)
 grouped_gemm_f64_kernel(const Tile* __restrict__ tiles, const Term* __restrict__ terms,
-                        const __grid_constant__ imps_dslots slots, double* ws, int* cnt) {
+                        const __grid_constant__ imps_planes planes, double* ws, int* cnt) {
   constexpr int RS = 32 * KI + 16, PL = TILE * RS;
   constexpr int NW = TILE / 8;  // warps per operand
   extern __shared__ __align__(16) unsigned char digits[];
@@ -233,6 +233,7 @@ grouped_gemm_f64_kernel(const Tile* __restrict__ tiles, const Term* __restrict__
   __shared__ int flags[2];  // of an even and an odd chunk
   __shared__ int last;
   imps::allow_successor();
+  const imps_dslots& slots = planes.s[blockIdx.y];
   if (threadIdx.x == 0) flags[0] = flags[1] = 0;
   __syncthreads();
   const Tile tl = tiles[blockIdx.x];
@@ -337,6 +338,8 @@ grouped_gemm_f64_kernel(const Tile* __restrict__ tiles, const Term* __restrict__
   if (tl.nparts > 1) {
     constexpr int WT = TILE * TILE / 4;  // threads that hold outputs
     // partial tile -> workspace; the last CTA of the tile sums all partials in share order
+    ws += blockIdx.y * planes.ws_len;
+    cnt += blockIdx.y * planes.cnt_len;
     double* wp = ws + ((int64_t)tl.ws_unit + tl.part) * (TILE * TILE) + threadIdx.x;
     if (writes)
 #pragma unroll
@@ -374,7 +377,7 @@ grouped_gemm_f64_kernel(const Tile* __restrict__ tiles, const Term* __restrict__
 template <int TILE>
 constexpr int smem_bytes(int ki) { return 2 * NS * TILE * (32 * ki + 16); }
 
-using KernelFn = void (*)(const Tile*, const Term*, imps_dslots, double*, int*);
+using KernelFn = void (*)(const Tile*, const Term*, imps_planes, double*, int*);
 template <int TILE>
 KernelFn kernel_of(int ki) {
   switch (ki) {
@@ -405,13 +408,21 @@ int imps_f64_setup() {
 
 int imps_launch_grouped_f64(const void* d_tiles, int ntiles, const void* d_terms, imps_dslots slots, int tile,
                             int ksteps, int splits, double* ws, int* cnt, void* stream) {
+  imps_planes one{};
+  one.s[0] = slots;
+  one.n = 1;
+  return imps_launch_grouped_f64(d_tiles, ntiles, d_terms, one, tile, ksteps, splits, ws, cnt, stream);
+}
+
+int imps_launch_grouped_f64(const void* d_tiles, int ntiles, const void* d_terms, const imps_planes& planes, int tile,
+                            int ksteps, int splits, double* ws, int* cnt, void* stream) {
   if (ntiles <= 0) return IMPS_OK;
-  if (splits < 1 || (splits > 1 && (!ws || !cnt)) || (tile != 16 && tile != 32)) return IMPS_ERR_BAD_ARG;
+  if (planes.n < 1 || planes.n > 2 || splits < 1 || (splits > 1 && (!ws || !cnt)) || (tile != 16 && tile != 32)) return IMPS_ERR_BAD_ARG;
   KernelFn fn = tile == 16 ? kernel_of<16>(ksteps) : kernel_of<32>(ksteps);
   if (!fn) return IMPS_ERR_BAD_ARG;
   imps::count_launch();
   const cudaError_t e =
-      imps::launch_overlapped(fn, dim3(ntiles), dim3(tile * 8), tile == 16 ? smem_bytes<16>(ksteps) : smem_bytes<32>(ksteps),
-                              (cudaStream_t)stream, (const Tile*)d_tiles, (const Term*)d_terms, slots, ws, cnt);
+      imps::launch_overlapped(fn, dim3(ntiles, planes.n), dim3(tile * 8), tile == 16 ? smem_bytes<16>(ksteps) : smem_bytes<32>(ksteps),
+                              (cudaStream_t)stream, (const Tile*)d_tiles, (const Term*)d_terms, planes, ws, cnt);
   return e == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
 }
