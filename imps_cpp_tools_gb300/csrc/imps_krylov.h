@@ -54,6 +54,9 @@ int kr_proj_epilogue(const double* x, const double* t, const double* s, const do
                      int64_t n, cudaStream_t st);
 int kr_trace_prod(const KrylovWs& ws, const double* X, const double* R, const int64_t* boff,
                   const int32_t* bdim, int nb, double* out, cudaStream_t st, const int32_t* bcols = nullptr);
+// A residual check's data in one overlapped kernel: copies and a synchronisation left the stream idle for
+// 14 us (Lanczos, three copies) to 24 us (GMRES, two) a check on this GPU.
+int kr_export(const double* src, int n, const int* f0, const int* f1, double* dst, int* dst_flags, cudaStream_t st);
 int kr_fac_epilogue(const double* ure, const double* uim, const double* tre, const double* tim, double c,
                     double s, const double* tau, const double* rho, double* ore, double* oim, int64_t n,
                     cudaStream_t st);

@@ -914,6 +914,24 @@ int kr_trace_prod(const KrylovWs& ws, const double* X, const double* R, const in
   return e == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
 }
 
+// n doubles and the flags f0, f1 (may be null) to pinned host memory
+__global__ void __launch_bounds__(256) export_kernel(const double* src, int n, const int* f0, const int* f1, double* dst,
+                                                     int* dst_flags) {
+  imps::allow_successor();
+  imps::wait_for_predecessor();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n) dst[t] = src[t];
+  if (t == 0) dst_flags[0] = f0 ? *f0 : 0;
+  if (t == 1) dst_flags[1] = f1 ? *f1 : 0;
+}
+
+int kr_export(const double* src, int n, const int* f0, const int* f1, double* dst, int* dst_flags, cudaStream_t st) {
+  imps::count_launch();
+  const cudaError_t e = imps::launch_overlapped(export_kernel, dim3(std::max(1, (n + 255) / 256)), dim3(256), 0, st, src, n,
+                                                f0, f1, dst, dst_flags);
+  return e == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
+}
+
 // out = u - fac * t + tau * rho on split complex planes (fac = c + i s; tau, rho optional):
 //   out_re = u_re - (c t_re - s t_im) + tau_re rho,  out_im = u_im - (s t_re + c t_im) + tau_im rho
 __global__ void fac_epilogue_kernel(const double* ure, const double* uim,
