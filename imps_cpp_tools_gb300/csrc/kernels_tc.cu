@@ -9,16 +9,20 @@
 //     packed[kstep][split][chunk][row group][8 rows][8 bf16]
 // so that the two K-steps of one pipeline stage are one contiguous bulk copy.
 //
-// Kernel roles (128 threads, one CTA per output tile of <= 128 x 128):
+// Kernel roles (256 threads, one CTA per output tile of <= 128 x 128):
 //   warp 0 lane 0 : producer, cp.async.bulk global -> shared, mbarrier complete_tx
 //   warp 1 lane 0 : MMA issuer, tcgen05.mma.cta_group::1.kind::f16 into TMEM, tcgen05.commit
-//   warps 0-3     : epilogue, tcgen05.ld 32x32b -> FP64 global
+//   warps 0-7     : epilogue, tcgen05.ld 32x32b -> FP64 global
 // Every mbarrier wait is bounded; on timeout the CTA records an error, drains what it
 // issued (bounded), frees its TMEM and returns.
 //
-// A tile is latency bound (a few dozen K steps), so two CTAs share an SM, the longest tiles start
-// first, and the kernels' launches overlap.  H_AC apply at Hubbard D = 1024 (209 tiles): 50.1 us with one
-// CTA of four pipeline stages per SM, table order, and the pack kernel's former stores; 28.4 now.
+// What bounds it: the chain of the longest tile, 40 K steps of 6 matrix instructions at 64 cycles each
+// whatever their N, some 270 cycles of barriers a stage, and the epilogue.  So two CTAs share an SM, the
+// longest tiles start first and the launches overlap; the issuing warp runs its loop as one (a lone lane spent
+// 830 cycles a K step, on descriptors, table reads and the abort flag; now 500); and eight warps write the
+// outputs, widened by integer operations at stepped pointers (11,400 -> 3,900 cycles for 96 columns).  A
+// operands hold their own rows only.  H_AC apply at Hubbard D = 1024 (209 tiles): 50.1 us with one CTA of
+// four stages per SM in table order and the pack kernel's former stores, 28.4 with two, 20.7 now.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -38,16 +42,13 @@ namespace {
 
 constexpr int TC_M = 128;        // UMMA M (rows of every tile, zero padded)
 constexpr int TC_NMAX = 128;     // max UMMA N per tile
-constexpr int TC_KSTAGE = 2;     // K-steps (of 16) per pipeline stage
-constexpr int TC_NSTAGE = 2;     // pipeline depth: two CTAs of two stages per SM, not one of four
-constexpr int TC_THREADS = 128;
-constexpr int A_STAGE_BYTES = TC_KSTAGE * 3 * TC_M * 32;     // 24 KB
-constexpr int B_STAGE_BYTES = TC_KSTAGE * 3 * TC_NMAX * 32;  // 24 KB
-constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
-// pipeline (2 x 48 KB) + alignment slack + headroom so that every descriptor-addressed access stays
-// inside this CTA's allocation; two CTAs fit an SM
+constexpr int TC_NSTAGE = 8;     // most pipeline stages
+constexpr int TC_THREADS = 256;
+constexpr int PIPE_BYTES = 98304;  // of the pipeline's stages
+// pipeline + alignment slack + headroom so that every descriptor-addressed access stays inside this
+// CTA's allocation; two CTAs fit an SM
 constexpr int SMEM_BYTES = 106496;  // 104 KB
-static_assert(TC_NSTAGE * STAGE_BYTES + 1024 <= SMEM_BYTES, "tcgen05 pipeline does not fit");
+static_assert(PIPE_BYTES + TC_M * 16 + 1024 <= SMEM_BYTES, "tcgen05 pipeline does not fit");
 constexpr uint32_t WAIT_LIMIT = 1u << 24;
 
 struct TcTerm {
@@ -61,7 +62,8 @@ struct TcTile {
   int32_t c_ld, m, n, npad;
   int32_t t0, t1;
   int16_t c_slot, accumulate;
-  int32_t pad;
+  int16_t mpad;             // rows of A as packed
+  int8_t kstage, nstage;    // K steps of a pipeline stage, stages
 };
 
 struct PackJob {
@@ -92,8 +94,9 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
                : "memory");
 }
 
-// bounded wait for the phase with the given parity; returns false on timeout
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+// bounded wait for the phase with the given parity; returns false on timeout, or once *abort is set (it is
+// looked at only while the phase is not there)
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const int* abort = nullptr) {
   const uint32_t a = smem_u32(bar);
   for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
     uint32_t ok;
@@ -103,8 +106,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
         : "r"(a), "r"(parity)
         : "memory");
     if (ok) return true;
+    if (abort && *(const volatile int*)abort) return false;
   }
   return false;
+}
+
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
+  return r != 0;
 }
 
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -213,6 +223,14 @@ __global__ void __launch_bounds__(256) pack_kernel(const PackJob* __restrict__ j
   }
 }
 
+// (double)x by integer operations where x is normal or zero: the conversion runs on the FP64 pipe, 64 cycles a
+// warp
+__device__ __forceinline__ double widen(float x) {
+  const uint32_t b = __float_as_uint(x), mag = b & 0x7fffffffu;
+  if (mag - 0x00800000u < 0x7f000000u) return __hiloint2double((int)((b & 0x80000000u) | ((mag >> 3) + 0x38000000u)), (int)(b << 29));
+  return mag == 0 ? __hiloint2double((int)b, 0) : (double)x;
+}
+
 __global__ void __launch_bounds__(TC_THREADS, 2)
 tc_gemm_kernel(const TcTile* __restrict__ tiles, const TcTerm* __restrict__ terms, const __nv_bfloat16* packed,
                const __grid_constant__ imps_dslots slots, int* err) {
@@ -225,7 +243,7 @@ tc_gemm_kernel(const TcTile* __restrict__ tiles, const TcTerm* __restrict__ term
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
   const TcTile tl = tiles[blockIdx.x];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t ncols = 128;  // TMEM columns (power of two >= npad)
   if (threadIdx.x == 0) {
     for (int s = 0; s < TC_NSTAGE; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -246,63 +264,83 @@ tc_gemm_kernel(const TcTile* __restrict__ tiles, const TcTerm* __restrict__ term
   imps::wait_for_predecessor();  // the packed operands are its predecessor's
   const int nterm = tl.t1 - tl.t0;
   const uint32_t idesc = idesc_bf16(TC_M, tl.npad);
-  const uint32_t a_split_bytes = TC_M * 32;          // one split of one K-step (A)
+  // one split of one K-step.  A holds mpad rows: the rows of an MMA past them read what follows in shared
+  // memory, and their outputs are not written
+  const uint32_t a_split_bytes = (uint32_t)tl.mpad * 32;
   const uint32_t b_split_bytes = (uint32_t)tl.npad * 32;
+  const int kstage = tl.kstage, nstage = tl.nstage;
+  const uint32_t a_stage_bytes = kstage * 3 * a_split_bytes, stage_bytes = a_stage_bytes + kstage * 3 * b_split_bytes;
+  int issued = 0;  // stages filled (by the producer)
 
   if (warp == 0 && lane == 0 && nterm > 0) {
     // ---------------- producer
     asm volatile("fence.proxy.async;" ::: "memory");  // the packs were written through the generic proxy
-    int it = 0;
+    int s = 0;
+    uint32_t u = 0;  // stage, and how often it has been filled before
     bool ok = true;
+    TcTerm next = terms[tl.t0];
+    const uint32_t a_step = 3 * a_split_bytes, b_step = 3 * b_split_bytes;  // of one K step
     for (int t = tl.t0; t < tl.t1 && ok; ++t) {
-      const TcTerm tm = terms[t];
-      for (int ks = 0; ks < tm.ksteps && ok; ks += TC_KSTAGE, ++it) {
-        const int s = it % TC_NSTAGE;
-        const uint32_t u = (uint32_t)(it / TC_NSTAGE);
-        if (u > 0 && !mbar_wait(&empty_bar[s], (u & 1) ^ 1)) { ok = false; break; }
-        if (*(volatile int*)&abort_s) { ok = false; break; }
-        const int nk = min(TC_KSTAGE, tm.ksteps - ks);
-        const uint32_t abytes = nk * 3 * a_split_bytes, bbytes = nk * 3 * b_split_bytes;
-        uint8_t* sa = smem + s * STAGE_BYTES;
-        uint8_t* sb = sa + A_STAGE_BYTES;
+      const TcTerm tm = next;
+      if (t + 1 < tl.t1) next = terms[t + 1];  // on its way meanwhile
+      const uint8_t* ga = (const uint8_t*)(packed + tm.a_off);
+      const uint8_t* gb = (const uint8_t*)(packed + tm.b_off);
+      for (int ks = 0; ks < tm.ksteps; ks += kstage) {
+        if (u > 0 && !mbar_wait(&empty_bar[s], (u & 1) ^ 1, &abort_s)) { ok = false; break; }
+        const int nk = min(kstage, tm.ksteps - ks);
+        const uint32_t abytes = nk * a_step, bbytes = nk * b_step;
+        uint8_t* sa = smem + s * stage_bytes;
+        uint8_t* sb = sa + a_stage_bytes;
         mbar_expect_tx(&full_bar[s], abytes + bbytes);
-        bulk_g2s(sa, packed + tm.a_off + (int64_t)ks * 3 * TC_M * 16, abytes, &full_bar[s]);
-        bulk_g2s(sb, packed + tm.b_off + (int64_t)ks * 3 * tl.npad * 16, bbytes, &full_bar[s]);
+        bulk_g2s(sa, ga, abytes, &full_bar[s]);
+        bulk_g2s(sb, gb, bbytes, &full_bar[s]);
+        ga += abytes;
+        gb += bbytes;
+        ++issued;
+        if (++s == nstage) { s = 0; ++u; }
       }
     }
     if (!ok) { atomicExch(err, 1); abort_s = 1; }
-  } else if (warp == 1 && lane == 0 && nterm > 0) {
-    // ---------------- MMA issuer
-    int it = 0;
-    uint32_t accum = 0;
+  } else if (warp == 1 && nterm > 0) {
+    // ---------------- MMA issuer: the whole warp runs the loop, one elected lane issues
+    const bool leader = elect_one();
+    const uint32_t a_step = a_split_bytes >> 4, b_step = b_split_bytes >> 4, stage_step = stage_bytes >> 4;
+    // descriptors of a stage's first core matrices; the others' lie whole multiples of a split further
+    const uint64_t ad0 = smem_desc(smem_u32(smem), tl.mpad * 16, 128);
+    const uint64_t bd0 = smem_desc(smem_u32(smem) + a_stage_bytes, tl.npad * 16, 128);
+    int s = 0, next = terms[tl.t0].ksteps;
+    uint32_t accum = 0, u = 0;
     bool ok = true;
     for (int t = tl.t0; t < tl.t1 && ok; ++t) {
-      const TcTerm tm = terms[t];
-      for (int ks = 0; ks < tm.ksteps; ks += TC_KSTAGE, ++it) {
-        const int s = it % TC_NSTAGE;
-        const uint32_t u = (uint32_t)(it / TC_NSTAGE);
-        if (!mbar_wait(&full_bar[s], u & 1) || *(volatile int*)&abort_s) { ok = false; break; }
+      const int ksteps = next;
+      if (t + 1 < tl.t1) next = terms[t + 1].ksteps;  // on its way meanwhile
+      for (int ks = 0; ks < ksteps; ks += kstage) {
+        if (!mbar_wait(&full_bar[s], u & 1, &abort_s)) { ok = false; break; }
         tc_fence_after();
-        const int nk = min(TC_KSTAGE, tm.ksteps - ks);
-        const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
-        const uint32_t sb = sa + A_STAGE_BYTES;
-        for (int k = 0; k < nk; ++k) {
-          // split pairs (a, b): hh, hm, mh, hl, mm, lh
-          const int pa[6] = {0, 0, 1, 0, 1, 2};
-          const int pb[6] = {0, 1, 0, 2, 1, 0};
-#pragma unroll
-          for (int q = 0; q < 6; ++q) {
-            const uint64_t ad = smem_desc(sa + (k * 3 + pa[q]) * a_split_bytes, TC_M * 16, 128);
-            const uint64_t bd = smem_desc(sb + (k * 3 + pb[q]) * b_split_bytes, tl.npad * 16, 128);
+        if (leader) {
+          const int nk = min(kstage, ksteps - ks);
+          uint64_t ad = ad0 + s * stage_step, bd = bd0 + s * stage_step;
+          for (int k = 0; k < nk; ++k, ad += 3 * a_step, bd += 3 * b_step) {
+            // split pairs (a, b): hh, hm, mh, hl, mm, lh
+            const uint64_t am = ad + a_step, al = am + a_step, bm = bd + b_step, bl = bm + b_step;
             mma_bf16(tmem, ad, bd, idesc, accum);
             accum = 1;
+            mma_bf16(tmem, ad, bm, idesc, 1);
+            mma_bf16(tmem, am, bd, idesc, 1);
+            mma_bf16(tmem, ad, bl, idesc, 1);
+            mma_bf16(tmem, am, bm, idesc, 1);
+            mma_bf16(tmem, al, bd, idesc, 1);
           }
+          mma_commit(&empty_bar[s]);  // frees the stage once these MMAs have read it
         }
-        mma_commit(&empty_bar[s]);  // frees the stage once these MMAs have read it
+        if (++s == nstage) { s = 0; ++u; }
       }
     }
-    if (!ok) { atomicExch(err, 1); abort_s = 1; }
-    mma_commit(&done_bar);  // arrives when every MMA issued above has completed
+    if (leader) {
+      if (!ok) { atomicExch(err, 1); abort_s = 1; }
+      mma_commit(&done_bar);  // arrives when every MMA issued above has completed
+    }
+    __syncwarp();
   }
   __syncthreads();  // role lanes rejoin their warps before the warp-collective TMEM loads
   // ---------------- epilogue
@@ -314,29 +352,34 @@ tc_gemm_kernel(const TcTile* __restrict__ tiles, const TcTerm* __restrict__ term
   }
   have = __all_sync(0xffffffffu, have);
   __syncwarp();
-  const int row = warp * 32 + lane;
-  for (int c0 = 0; c0 < tl.npad; c0 += 16) {
+  // warps w and w + 4 take the rows of TMEM lanes 32 (w % 4) .., every other 16 columns each
+  const int row = (warp & 3) * 32 + lane;
+  const bool acc = tl.accumulate != 0;
+  const int64_t ldc = tl.c_ld;
+  double* p = C + row + (warp >> 2) * 16 * ldc;
+  for (int c0 = (warp >> 2) * 16; c0 < tl.npad; c0 += 32) {
     float v[16];
     if (have) {
-      tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
+      tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
     } else {
 #pragma unroll
       for (int i = 0; i < 16; ++i) v[i] = 0.f;
     }
     if (row < tl.m) {
+      if (!acc && c0 + 16 <= tl.n) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const int col = c0 + i;
-        if (col < tl.n) {
-          double* p = C + row + (int64_t)col * tl.c_ld;
-          *p = tl.accumulate ? *p + (double)v[i] : (double)v[i];
-        }
+        for (int i = 0; i < 16; ++i) p[i * ldc] = widen(v[i]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (c0 + i < tl.n) p[i * ldc] = acc ? p[i * ldc] + widen(v[i]) : widen(v[i]);
       }
     }
+    p += 32 * ldc;
   }
   // producer drains its copies if it aborted (bounded), then TMEM is released
   if (warp == 0 && lane == 0 && abort_s) {
-    for (int s = 0; s < TC_NSTAGE; ++s) mbar_wait(&full_bar[s], 0);
+    for (int i = max(0, issued - nstage); i < issued; ++i) mbar_wait(&full_bar[i % nstage], (i / nstage) & 1);
   }
   tc_fence_before();
   __syncthreads();
@@ -407,6 +450,11 @@ int tc_create(TcPlan** out, const Plan& P, cudaStream_t st) {
           tl.m = std::min(TC_M, o.M - m0);
           tl.n = std::min(TC_NMAX, o.N - n0);
           tl.npad = std::max(16, round_up(tl.n, 16));
+          tl.mpad = (int16_t)std::max(8, round_up(tl.m, 8));
+          // two K steps a stage (one: 18.4 us for the kernel at Hubbard D = 1024 instead of 16.1, as a stage
+          // costs its barriers some 270 cycles), as many stages as fit: 2 of 128 x 128 to 8 of 48 x 16
+          tl.kstage = 2;
+          tl.nstage = (int8_t)std::min(TC_NSTAGE, PIPE_BYTES / (tl.kstage * 3 * 32 * (tl.mpad + tl.npad)));
           tl.c_slot = o.c_slot;
           tl.accumulate = o.accumulate;
           tl.t0 = (int)ts.terms.size();
@@ -417,7 +465,7 @@ int tc_create(TcPlan** out, const Plan& P, cudaStream_t st) {
             std::vector<PackJob>& ja = T->dynamic_slot[tm.a_slot] ? ts.dyn_jobs : T->static_jobs;
             std::vector<PackJob>& jb = T->dynamic_slot[tm.b_slot] ? ts.dyn_jobs : T->static_jobs;
             TcTerm tt{};
-            tt.a_off = pack_for(tm.a_slot, tm.a_off, tm.a_ld, tm.a_t, 0, m0, tl.m, tm.k, TC_M, tm.alpha, ja);
+            tt.a_off = pack_for(tm.a_slot, tm.a_off, tm.a_ld, tm.a_t, 0, m0, tl.m, tm.k, tl.mpad, tm.alpha, ja);
             tt.b_off = pack_for(tm.b_slot, tm.b_off, tm.b_ld, tm.b_t, 1, n0, tl.n, tm.k, tl.npad, 1.0, jb);
             tt.ksteps = round_up(tm.k, 16) / 16;
             ts.terms.push_back(tt);
