@@ -192,7 +192,9 @@ __device__ void apply_reflectors(const double* a, int M, int K, const double* ta
 // of each column is the longer part: some 6,000 cycles for dot product, update, norm, square root and
 // division, 1,300 to read the reflector from another SM, 600 to arrive at the barrier.  The norm is
 // taken from the updated column: from the old one's sums it costs a reduction less, but cancels (2.9e-13
-// off for 1.2e-15) and was no faster.  QR of A_C and C at Hubbard D = 1024: 3,420 -> 904 us.
+// off for 1.2e-15) and was no faster.  The maker's other warps wait until it is done: sharing the FP64 pipe
+// they delayed the reflector that every CTA needs next (875 us; 818 so), and their CTA has the next seven steps to
+// catch up.  QR of A_C and C at Hubbard D = 1024: 3,420 -> 818 us.
 constexpr int QC = 8;      // CTAs per cluster (the portable maximum)
 constexpr int QT = 256;    // threads per CTA
 constexpr int QR_SMEM = 200 * 1024;
@@ -315,10 +317,9 @@ qr_cluster_kernel(const imps::DenseMat* __restrict__ mats, const double* __restr
     }
     __syncwarp();
     if (k + 1 < N) cluster_arrive();
-    if (!maker && tau != 0.0) {
-      const int w0 = next ? warp - 4 : warp, nw = next ? 4 : QT / 32;
-      for (int jl = first + (next ? 1 : 0) + w0; jl < mine; jl += nw) reflect(cols + (size_t)jl * M, v, tau, M, k, lane);
-    }
+    if (next) __syncthreads();  // the FP64 pipe is the maker's until reflector k + 1 is made
+    if (tau != 0.0)
+      for (int jl = first + (next ? 1 : 0) + warp; jl < mine; jl += QT / 32) reflect(cols + (size_t)jl * M, v, tau, M, k, lane);
   }
   __syncthreads();
   // R (N x N) with a non-negative diagonal: row i times sgn_i
