@@ -52,9 +52,10 @@ METRIC = "VUMPS sweeps/s + H_AC TFLOP/s, mixed vs FP64 on one GB300 at |dE|<=1e-
 APPLIES_PER_STEP = 20
 L2_FLUSH_BYTES = 512 << 20
 # DRAM bytes (read + write) of one H_AC apply from one ncu capture of `bench.py --mode hac`
-# (profiles/tc_gemm_hac_xxz_d512.md: tc_gemm 5.26 MB + pack 0.40 MB;
-# profiles/grouped_gemm_f64_hac_xxz_d512.md, autotuned shape 16x16 split 2: 2.38 + 0.03 MB)
-NCU_TRAFFIC_BYTES = {"bf16x6": 5.66e6, "fp64": 2.41e6}
+# (profiles/tc_gemm_hac_xxz_d512.md: tc_gemm 2.73 MB, and 0.40 MB of the pack's input;
+# profiles/grouped_gemm_f64_hac_xxz_d512.md, autotuned shape 32x32 with 4 shares: 2.39 MB)
+NCU_TRAFFIC_BYTES = {"bf16x6": 3.13e6, "fp64": 2.39e6}
+FP16_DIGIT_PRODUCTS = 28
 # tolerances of the timed sweeps: the eigensolver tolerance of the configuration (1e-12); GMRES
 # 1e-8, because the environment systems of these states do not reach 1e-12 in floating point:
 # measured at XXZ D=512 from the warmed state, the relative residual of the left-environment
@@ -509,8 +510,8 @@ def run_vumps(args):
             "flops_per_apply": flops, "fp64_us": t_hac64 * 1e6, "mixed_us": t_hacmx * 1e6,
             "fp64_launch_shape": {"tile": tile, "splits": splits,
                                   "source": "autotuner" if _AUTOTUNE[0] else "makespan estimate"}}
-    fp64_src = ("dense FP64 matmul (torch, cuBLAS DGEMM 4096^3) measured in this run: GB300 has no FP64 tensor "
-                "rate, the FP64 pipe bounds this kernel (not in MEASURED_PEAKS.json)")
+    fp64_src = ("dense FP64 matmul (torch, cuBLAS DGEMM 4096^3) measured in this run (not in MEASURED_PEAKS.json); "
+                "no bound of this kernel, whose FP64 products are formed from FP16 digits on the tensor pipe")
     if args.precision == "bf16x6":
         achieved = 6 * flops / t_hacmx / 1e12
         roof = {"bound": "tensor", "achieved": achieved, "peak": bf16_peak, "unit": "TFLOP/s",
@@ -521,10 +522,15 @@ def run_vumps(args):
                 "fp64_engine": {"achieved": flops / t_hac64 / 1e12, "peak": fp64_peak,
                                 "frac": flops / t_hac64 / 1e12 / fp64_peak, "peak_source": fp64_src}}
     else:
-        achieved = flops / t_hac64 / 1e12
-        roof = {"bound": "fp64_pipe", "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
-                "frac": achieved / fp64_peak, "traffic": NCU_TRAFFIC_BYTES["fp64"], "peak_source": fp64_src,
-                "kernel": "grouped_gemm_f64 (H_AC apply; the dominant kernel of the timed sweeps)",
+        achieved = FP16_DIGIT_PRODUCTS * flops / t_hac64 / 1e12
+        roof = {"bound": "tensor", "achieved": achieved, "peak": bf16_peak, "unit": "TFLOP/s",
+                "frac": achieved / bf16_peak, "traffic": NCU_TRAFFIC_BYTES["fp64"],
+                "peak_source": "MEASURED_PEAKS.json bf16_tflops (burst), of measured; mma.sync, which this kernel "
+                               "issues, reaches about a third of it on this GPU",
+                "kernel": "grouped_gemm_f64 (H_AC apply; 28 FP16 digit products per FP64 product; the dominant kernel "
+                          "of the timed sweeps)",
+                "fp64_equivalent": {"achieved": flops / t_hac64 / 1e12, "peak": fp64_peak,
+                                    "frac": flops / t_hac64 / 1e12 / fp64_peak, "peak_source": fp64_src},
                 "split_bf16_engine": {"achieved_fp64_equivalent_tflops": flops / t_hacmx / 1e12,
                                       "tensor_tflops": 6 * flops / t_hacmx / 1e12, "tensor_peak": bf16_peak,
                                       "tensor_frac": 6 * flops / t_hacmx / 1e12 / bf16_peak}}
