@@ -1099,8 +1099,9 @@ static int eigs_impl(imps_ctx* c, imps_plan* p, int64_t n, const DevApply& op, d
   if (kk >= m) return IMPS_ERR_BAD_ARG;
   const bool cb_arena = p == nullptr;  // operator is a callback: keep clear of its solvers
   RC(arena_reserve(c, round256(n * 8) * (m + 4 + kk) + round256((size_t)ld * ld * 8) +
-                          round256((size_t)m * kk * 8) + 4096, cb_arena));
+                          round256((size_t)m * kk * 8) + round256(kr_rotate_scratch(n, kk)) + 4096, cb_arena));
   Bump bp{cb_arena ? c->arena_cb : c->arena};
+  double* rot = bp.take(kr_rotate_scratch(n, kk) / 8);
   double* V = bp.take((size_t)n * (m + 1));
   double* Wk = bp.take((size_t)n * kk);
   double* w = bp.take(n);
@@ -1249,7 +1250,7 @@ static int eigs_impl(imps_ctx* c, imps_plan* p, int64_t n, const DevApply& op, d
       }
       std::copy(Wr.begin(), Wr.end(), c->hpin);  // pinned: the upload is asynchronous
       CK(cudaMemcpyAsync(Wrot, c->hpin, (size_t)m * kk * 8, cudaMemcpyHostToDevice, st));
-      RC(kr_basis_rotate(V, n, m, Wrot, kk, Wk, n, n, st));
+      RC(kr_basis_rotate(V, n, m, Wrot, kk, Wk, n, n, rot, st));
       CK(cudaMemcpyAsync(V, Wk, (size_t)kk * n * 8, cudaMemcpyDeviceToDevice, st));
       CK(cudaMemcpyAsync(V + (size_t)kk * n, V + (size_t)m * n, n * 8, cudaMemcpyDeviceToDevice, st));
       for (int pc = 0; pc < kk; ++pc) ta[pc] = qa[kk - 1 - pc];
@@ -1267,7 +1268,7 @@ static int eigs_impl(imps_ctx* c, imps_plan* p, int64_t n, const DevApply& op, d
       CK(cudaStreamSynchronize(st));
       std::copy(Zv.begin(), Zv.begin() + (size_t)kfinal * nev, c->hpin);
       CK(cudaMemcpyAsync(Wrot, c->hpin, (size_t)kfinal * nev * 8, cudaMemcpyHostToDevice, st));
-      RC(kr_basis_rotate(V, n, kfinal, Wrot, nev, evecs, n, n, st));
+      RC(kr_basis_rotate(V, n, kfinal, Wrot, nev, evecs, n, n, rot, st));
     }
     CK(cudaStreamSynchronize(st));
     return status;
@@ -1355,8 +1356,9 @@ int imps_eigs_rs_batch_op(imps_ctx* c, int P, int64_t n, imps_apply_fn fn, void*
                           round256((size_t)P * n * 8) * 2 + round256((size_t)P * ld * ld * 8) +
                           round256((size_t)m * kk * 8) + round256(ld * 8) + 2 * round256((size_t)P * 8) +
                           round256((size_t)P * kMaxCols * 8) + round256((size_t)P * CGS_BATCH_GRID * kMaxCols * 8) +
-                          4096, true));
+                          round256(kr_rotate_scratch(n, kk)) + 4096, true));
   Bump bp{c->arena_cb};
+  double* rot = bp.take(kr_rotate_scratch(n, kk) / 8);
   double* V = bp.take((size_t)P * n * (m + 1));  // system s: V + s * n * (m + 1), column j at + j * n
   double* Wk = bp.take((size_t)n * kk);
   double* IN = bp.take((size_t)P * n);
@@ -1497,7 +1499,7 @@ int imps_eigs_rs_batch_op(imps_ctx* c, int P, int64_t n, imps_apply_fn fn, void*
         }
       }
       CK(cudaMemcpy(Wrot, Wr.data(), (size_t)m * kk * 8, cudaMemcpyHostToDevice));
-      RC(kr_basis_rotate(Vs(sy), n, m, Wrot, kk, Wk, n, n, st));
+      RC(kr_basis_rotate(Vs(sy), n, m, Wrot, kk, Wk, n, n, rot, st));
       CK(cudaMemcpyAsync(Vs(sy), Wk, (size_t)kk * n * 8, cudaMemcpyDeviceToDevice, st));
       CK(cudaMemcpyAsync(Vs(sy) + (size_t)kk * n, Vs(sy) + (size_t)m * n, n * 8, cudaMemcpyDeviceToDevice, st));
       CK(cudaStreamSynchronize(st));  // Wrot and Wk are reused by the next system
@@ -1541,8 +1543,9 @@ static int eign_impl(imps_ctx* c, imps_plan* p, int64_t n, const DevApply& op, c
   const int ld = m + 1;
   const bool cb_arena = p == nullptr;
   RC(arena_reserve(c, round256(n * 8) * (2 * (size_t)m + 3) + round256((size_t)ld * ld * 8) +
-                          round256((size_t)m * m * 8) + 4096, cb_arena));
+                          round256((size_t)m * m * 8) + round256(kr_rotate_scratch(n, m)) + 4096, cb_arena));
   Bump bp{cb_arena ? c->arena_cb : c->arena};
+  double* rot = bp.take(kr_rotate_scratch(n, m) / 8);
   double* V = bp.take((size_t)n * (m + 1));
   double* Wk = bp.take((size_t)n * m);
   double* w = bp.take(n);
@@ -1689,7 +1692,7 @@ static int eign_impl(imps_ctx* c, imps_plan* p, int64_t n, const DevApply& op, c
     for (int b = 0; b < q; ++b)
       for (int r = 0; r < k; ++r) c->hpin[r + (size_t)b * k] = Qh[r + (size_t)b * m];
     CK(cudaMemcpyAsync(Qd, c->hpin, (size_t)k * q * 8, cudaMemcpyHostToDevice, st));
-    RC(kr_basis_rotate(V, n, k, Qd, q, Wk, n, n, st));
+    RC(kr_basis_rotate(V, n, k, Qd, q, Wk, n, n, rot, st));
     CK(cudaMemcpyAsync(V, Wk, (size_t)q * n * 8, cudaMemcpyDeviceToDevice, st));
     CK(cudaMemcpyAsync(V + (size_t)q * n, V + (size_t)m * n, n * 8, cudaMemcpyDeviceToDevice, st));
     std::fill(G.begin(), G.end(), 0.0);
@@ -1717,10 +1720,10 @@ static int eign_impl(imps_ctx* c, imps_plan* p, int64_t n, const DevApply& op, c
         }
       CK(cudaMemcpyAsync(Qd, c->hpin, (size_t)k * nout * 8, cudaMemcpyHostToDevice, st));
       if (mem == IMPS_MEM_HOST) {
-        RC(kr_basis_rotate(V, n, k, Qd, nout, Wk, n, n, st));
+        RC(kr_basis_rotate(V, n, k, Qd, nout, Wk, n, n, rot, st));
         CK(cudaMemcpyAsync(dst, Wk, (size_t)nout * n * 8, cudaMemcpyDeviceToHost, st));
       } else {
-        RC(kr_basis_rotate(V, n, k, Qd, nout, dst, n, n, st));
+        RC(kr_basis_rotate(V, n, k, Qd, nout, dst, n, n, rot, st));
       }
       CK(cudaStreamSynchronize(st));
     }

@@ -188,8 +188,9 @@ struct imps_planes {
 int imps_f64_setup();
 int imps_launch_grouped_f64(const void* d_tiles, int ntiles, const void* d_terms, imps_dslots slots, int tile,
                             int ksteps, int splits, double* ws, int* cnt, void* stream);
+// after_tables: the launch before this one writes the tables, which an overlapped launch would read too early
 int imps_launch_grouped_f64(const void* d_tiles, int ntiles, const void* d_terms, const imps_planes& planes, int tile,
-                            int ksteps, int splits, double* ws, int* cnt, void* stream);
+                            int ksteps, int splits, double* ws, int* cnt, void* stream, bool after_tables = false);
 
 #ifdef __CUDACC__
 // ----- overlapped launches -----

@@ -415,14 +415,19 @@ int imps_launch_grouped_f64(const void* d_tiles, int ntiles, const void* d_terms
 }
 
 int imps_launch_grouped_f64(const void* d_tiles, int ntiles, const void* d_terms, const imps_planes& planes, int tile,
-                            int ksteps, int splits, double* ws, int* cnt, void* stream) {
+                            int ksteps, int splits, double* ws, int* cnt, void* stream, bool after_tables) {
   if (ntiles <= 0) return IMPS_OK;
   if (planes.n < 1 || planes.n > 2 || splits < 1 || (splits > 1 && (!ws || !cnt)) || (tile != 16 && tile != 32)) return IMPS_ERR_BAD_ARG;
   KernelFn fn = tile == 16 ? kernel_of<16>(ksteps) : kernel_of<32>(ksteps);
   if (!fn) return IMPS_ERR_BAD_ARG;
   imps::count_launch();
-  const cudaError_t e =
-      imps::launch_overlapped(fn, dim3(ntiles, planes.n), dim3(tile * 8), tile == 16 ? smem_bytes<16>(ksteps) : smem_bytes<32>(ksteps),
-                              (cudaStream_t)stream, (const Tile*)d_tiles, (const Term*)d_terms, planes, ws, cnt);
+  const int smem = tile == 16 ? smem_bytes<16>(ksteps) : smem_bytes<32>(ksteps);
+  if (after_tables) {
+    fn<<<dim3(ntiles, planes.n), dim3(tile * 8), smem, (cudaStream_t)stream>>>((const Tile*)d_tiles, (const Term*)d_terms, planes,
+                                                                               ws, cnt);
+    return cudaGetLastError() == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
+  }
+  const cudaError_t e = imps::launch_overlapped(fn, dim3(ntiles, planes.n), dim3(tile * 8), smem, (cudaStream_t)stream,
+                                                (const Tile*)d_tiles, (const Term*)d_terms, planes, ws, cnt);
   return e == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
 }

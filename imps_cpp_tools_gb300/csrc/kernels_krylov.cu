@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <limits>
 
 #include "imps_krylov.h"
 #include "imps_status.h"
@@ -544,47 +545,36 @@ __global__ void gemv_kernel(const double* __restrict__ V, int64_t ldv, int ncols
 }
 
 // y = x / *nrm  (guarded: a zero norm writes zeros and raises the breakdown flag)
-// out[:, t] = sum_i V[:, i] * W[i + t*m] for t < kk (column-major W, m <= kMaxCols): the
-// basis rotation of a thick restart, one pass over V per 16 output columns (V stays in L2).
-__global__ void __launch_bounds__(256) basis_rotate_kernel(const double* __restrict__ V, int64_t ldv,
-                                                           int m, const double* __restrict__ W, int kk,
-                                                           double* __restrict__ out, int64_t ldo,
-                                                           int64_t n) {
-  constexpr int CT = 16;
-  __shared__ double ws[imps::kMaxCols * CT];
-  for (int t0 = 0; t0 < kk; t0 += CT) {
-    const int nt = min(CT, kk - t0);
-    __syncthreads();
-    for (int e = threadIdx.x; e < m * CT; e += blockDim.x) {
-      const int i = e / CT, t = e % CT;
-      ws[e] = t < nt ? W[i + (int64_t)(t0 + t) * m] : 0.0;
-    }
-    __syncthreads();
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n;
-         r += (int64_t)gridDim.x * blockDim.x) {
-      double acc[CT];
-#pragma unroll
-      for (int t = 0; t < CT; ++t) acc[t] = 0.0;
-      int i = 0;
-      for (; i + 8 <= m; i += 8) {  // eight loads in flight per thread
-        double v[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = V[r + (int64_t)(i + q) * ldv];
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-#pragma unroll
-          for (int t = 0; t < CT; ++t) acc[t] = fma(v[q], ws[(i + q) * CT + t], acc[t]);
-      }
-      for (; i < m; ++i) {
-        const double v = V[r + (int64_t)i * ldv];
-#pragma unroll
-        for (int t = 0; t < CT; ++t) acc[t] = fma(v, ws[i * CT + t], acc[t]);
-      }
-#pragma unroll
-      for (int t = 0; t < CT; ++t)
-        if (t < nt) out[r + (int64_t)(t0 + t) * ldo] = acc[t];
-    }
+// The tables of one block out (n x kk) = V (n x m) W (m x kk) for the grouped GEMM: slots 2, 0, 1, 32 x 32 tiles,
+// one term.  A thick restart's rotation is a contraction, so it belongs there (split FP16 digits on the tensor
+// cores) and not on the FP64 pipe, whose bound a kernel of its own reached: 48,066 x 126 by 63 columns 1,010
+// -> 113 us, by 1 column 256 -> 47; 2,000 x 32 by 16 38 -> 8; 150,276 x 126 by 63 2,015 -> 338.
+__global__ void rotate_tables_kernel(imps::Term* term, imps::Tile* tiles, int rows, int cols, int n, int ldv, int ldo, int m, int kk,
+                                     int kc) {
+  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  if (id == 0) {
+    imps::Term t{};
+    t.a_slot = 0;
+    t.a_ld = ldv;
+    t.b_slot = 1;
+    t.b_ld = m;
+    t.k = m;
+    t.kc = (int16_t)kc;
+    t.alpha = 1.0;
+    *term = t;
   }
+  if (id >= rows * cols) return;
+  imps::Tile t{};
+  t.c_ld = ldo;
+  t.c_slot = 2;
+  t.m0 = id % rows * 32;
+  t.n0 = id / rows * 32;
+  t.mt = min(32, n - t.m0);
+  t.nt = min(32, kk - t.n0);
+  t.t1 = 1;
+  t.nparts = 1;
+  t.nch = (m + kc - 1) / kc;
+  tiles[id] = t;
 }
 
 __global__ void scale_inv_kernel(const double* __restrict__ x, const double* __restrict__ nrm,
@@ -803,12 +793,33 @@ int kr_gemv(const double* V, int64_t ldv, int ncols, const double* h, double* y,
   return IMPS_OK;
 }
 
+size_t kr_rotate_scratch(int64_t n, int kk) {
+  return 64 + (size_t)((n + 31) / 32) * ((kk + 31) / 32) * sizeof(Tile);
+}
+
 int kr_basis_rotate(const double* V, int64_t ldv, int m, const double* W, int kk, double* out,
-                    int64_t ldo, int64_t n, cudaStream_t st) {
+                    int64_t ldo, int64_t n, void* scratch, cudaStream_t st) {
   if (m < 1 || m > kMaxCols || kk < 1 || n < 1) return IMPS_ERR_BAD_ARG;
+  const int64_t most = std::numeric_limits<int32_t>::max() - 31;  // the tables' row numbers and leading dimensions
+  if (n > most || ldv > most || ldo > most) {
+    for (int t = 0; t < kk; ++t) {
+      const int rc = kr_gemv(V, ldv, m, W + (size_t)t * m, out + (size_t)t * ldo, n, st);
+      if (rc) return rc;
+    }
+    return IMPS_OK;
+  }
+  const int rows = (int)((n + 31) / 32), cols = (kk + 31) / 32, kc = chunk_len(m);
+  Tile* tiles = (Tile*)((char*)scratch + 64);
   imps::count_launch();
-  basis_rotate_kernel<<<grid_for(n), 256, 0, st>>>(V, ldv, m, W, kk, out, ldo, n);
-  return IMPS_OK;
+  rotate_tables_kernel<<<(rows * cols + 255) / 256, 256, 0, st>>>((Term*)scratch, tiles, rows, cols, (int)n, (int)ldv, (int)ldo, m,
+                                                                  kk, kc);
+  if (cudaGetLastError() != cudaSuccess) return IMPS_ERR_CUDA;
+  imps_planes pl{};
+  pl.n = 1;
+  pl.s[0].p[0] = const_cast<double*>(V);
+  pl.s[0].p[1] = const_cast<double*>(W);
+  pl.s[0].p[2] = out;
+  return imps_launch_grouped_f64(tiles, rows * cols, scratch, pl, 32, kc / 16, 1, nullptr, nullptr, st, true);
 }
 
 int kr_cgs2_step(const KrylovWs& ws, const double* V, int64_t ldv, int nc, double* w, int64_t n,
