@@ -624,8 +624,9 @@ __device__ int jacobi_sweeps(T* B, T* V, int N, int ld, double tol, int max_swee
 }
 
 // SVD of the M x N sector matrix held in U (M >= N, N <= kJacobiMaxN) by one CTA, for sectors whose columns
-// do not fit a cluster's shared memory (N = 96: M > 1,470), with the preconditioning of Drmac and Veselic (SIAM J. Matrix Anal. Appl. 29 (2008) 1322): Householder
-// QR with column pivoting A P = Q R, then one-sided Jacobi on the columns of X = R^T, which is
+// do not fit a cluster's shared memory (N = 96: M > 1,470), with the preconditioning of Drmac and Veselic
+// (SIAM J. Matrix Anal. Appl. 29 (2008) 1322): Householder QR with column pivoting A P = Q R, then one-sided
+// Jacobi on the columns of X = R^T, which is
 // strongly graded and converges in a few sweeps (the unpivoted form needs 15-30 sweeps on
 // sectors whose singular values span many decades).  X Vx = Ux S gives R = Vx S Ux^T, so
 // U = Q [Vx; 0] and V = P Ux.  MIXED: the first sweeps run in FP32 (many times the FP64 rate
