@@ -199,8 +199,21 @@ constexpr int QC = 8;      // CTAs per cluster (the portable maximum)
 constexpr int QT = 256;    // threads per CTA
 constexpr int QR_SMEM = 200 * 1024;
 
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// An .aligned barrier wants the whole warp at it together, and what comes before may leave its lanes apart (a
+// loop over rows ends for some lanes before others, lane 0 stores alone): __syncwarp() brings them back.
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the same for warps 0-3 alone (bar.sync is the aligned form)
+__device__ __forceinline__ void sync128() {
+  __syncwarp();
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+}
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -221,7 +234,7 @@ __device__ __forceinline__ double sum128(double v, double* sh, int half) {
   v = wsum(v);
   double* s = sh + 4 * half;
   if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
-  asm volatile("bar.sync 1, 128;" ::: "memory");
+  sync128();
   return (s[0] + s[1]) + (s[2] + s[3]);
 }
 
@@ -239,7 +252,7 @@ __device__ void make_reflector(double* x, int M, int k, double tail, double* tau
     t = __shfl_sync(0xffffffffu, q, 0);
     scal = __shfl_sync(0xffffffffu, q, 1);
   }
-  asm volatile("bar.sync 1, 128;" ::: "memory");  // x[k] has been read
+  sync128();  // x[k] has been read
   if (t != 0.0)
     for (int i = k + 1 + (int)threadIdx.x; i < M; i += 128) x[i] *= scal;
   if (threadIdx.x == 0) {
@@ -315,7 +328,6 @@ qr_cluster_kernel(const imps::DenseMat* __restrict__ mats, const double* __restr
       }
       make_reflector(c, M, k + 1, tail, tau_s + k + 1, beta_s + k + 1, sh);
     }
-    __syncwarp();
     if (k + 1 < N) cluster_arrive();
     if (next) __syncthreads();  // the FP64 pipe is the maker's until reflector k + 1 is made
     if (tau != 0.0)
@@ -804,7 +816,6 @@ __host__ __device__ constexpr size_t svd_work_doubles(int M, int N, int kc, bool
 }
 
 __device__ __forceinline__ void cluster_sync() {
-  __syncwarp();
   cluster_arrive();
   cluster_wait();
 }
@@ -1359,7 +1370,6 @@ svd_cluster_kernel(const imps::SvdSets sets, int smem_doubles, int max_sweeps, i
       for (int jl = warp; jl < mine; jl += nw) reflect(uc + jl * ldu, vbuf + (size_t)(k & 1) * M, tau_s[k], M, k, lane);
     __syncthreads();
   }
-  __syncwarp();
   cluster_arrive();
   if (u_shared)
     for (int jl = warp; jl < mine; jl += nw)

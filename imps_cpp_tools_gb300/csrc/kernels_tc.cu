@@ -252,6 +252,7 @@ tc_gemm_kernel(const TcTile* __restrict__ tiles, const TcTerm* __restrict__ term
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
+    __syncwarp();  // thread 0 comes from the barriers' initialisation
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)),
                  "r"(ncols)
                  : "memory");
@@ -384,6 +385,7 @@ tc_gemm_kernel(const TcTile* __restrict__ tiles, const TcTerm* __restrict__ term
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
   }
 }
