@@ -153,6 +153,20 @@ static int max_chunks(const Stage& S) {
 
 static int max_splits(const Stage& S) { return std::max(1, std::min(8, max_chunks(S))); }
 
+// The terms in the order of the device's sums: of each block every other one, then those between.  Neighbours
+// are alike (H_AC: the two environments, then the reduced operators), and where they need plain FP64
+// (kernels_f64.cu) no share of a sum should get them all: H_AC at XXZ D = 512 with both environment terms in
+// plain FP64 takes 72 us, 114 in the table's order.
+static std::vector<Term> device_terms(const Stage& S) {
+  std::vector<Term> out = S.terms;
+  for (const OutBlock& o : S.outs) {
+    int at = o.t0;
+    for (int first = 0; first < 2; ++first)
+      for (int t = o.t0 + first; t < o.t1; t += 2) out[at++] = S.terms[t];
+  }
+  return out;
+}
+
 // (re)build the stage's tiles for shape (T, splits) and upload them.  Split-K in proportion to
 // the work: the tile with the most K chunks is split over `splits` CTAs, every other tile over
 // ceil(splits x its chunks / the most chunks), so that the CTAs of a launch carry about equal
@@ -162,6 +176,7 @@ static int install_stage(Stage& S, int T, int splits) {
   S.d_tiles = nullptr; S.d_ws = nullptr; S.d_cnt = nullptr;
   finalize_tiles(S, T, T);
   S.splits = splits;
+  const std::vector<Term> terms = device_terms(S);
   const size_t ntiles = S.tiles.size();
   int cmax = 1;
   for (const Tile& t : S.tiles) cmax = std::max(cmax, t.nch);
@@ -184,7 +199,7 @@ static int install_stage(Stage& S, int T, int splits) {
       t.t0 = term;
       t.c0 = chunk;
       for (int c = 0; c < t.nch;) {
-        const int left = num_chunks(S.terms[term].k) - chunk;
+        const int left = num_chunks(terms[term].k) - chunk;
         if (left <= t.nch - c) { c += left; ++term; chunk = 0; }
         else { chunk += t.nch - c; c = t.nch; }
       }
@@ -210,11 +225,11 @@ static int install_stage(Stage& S, int T, int splits) {
 }
 
 // Launch shape by estimate.  Tile edge 16 where 32 x 32 tiles would give fewer than one K chunk per
-// SM (a transfer-matrix stage at XXZ D = 512: 9.1 us with 16, 10.3 with 32; with more chunks the
-// fourfold splitting of the operands costs more than it spreads: H_AC at XXZ D = 512 18.5 us with 32,
-// 22.5 with 16, at Hubbard D = 1024 45 and 66).  Shares of as many chunks as leave about three CTAs
-// per SM: H_AC at XXZ D = 512 28.7 us unsplit, 17.8 to 18.7 with 3 to 8 shares; at Hubbard D = 1024
-// 56 unsplit, 49 with 2 or 4, 53 with 8.
+// SM (the four transfer-matrix stages at XXZ D = 512: 35.2 us with 16, 40.4 with 32; with more chunks the
+// fourfold splitting of the operands costs more than it spreads: H_AC at XXZ D = 512 19.0 us with 32,
+// 20.9 with 16, at Hubbard D = 1024 47.7 and 71.2).  Shares of as many chunks as leave about three CTAs
+// per SM: H_AC at XXZ D = 512 42.5 us unsplit, 18.9 with 3 or 4 shares, 17.6 with 8; at Hubbard D = 1024
+// 66.9 unsplit, 47.5 to 48.0 with 2 to 4, 52.4 with 8.
 static void shape_estimate(const Stage& S, int* T, int* splits) {
   constexpr int kSMs = 152;
   int64_t units = 0;
@@ -242,7 +257,7 @@ int upload_stage(Stage& S) {
   RC(install_stage(S, T, sp));
   if (!S.terms.empty()) {
     CK(cudaMalloc(&S.d_terms, S.terms.size() * sizeof(Term)));
-    CK(cudaMemcpy(S.d_terms, S.terms.data(), S.terms.size() * sizeof(Term), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(S.d_terms, device_terms(S).data(), S.terms.size() * sizeof(Term), cudaMemcpyHostToDevice));
   }
   return IMPS_OK;
 }

@@ -68,8 +68,9 @@ struct Tile {
   int16_t c_slot;
   int16_t accumulate;  // 1: C += sum, 0: C = sum
   // split-K: the CTA of this entry takes share `part` of `nparts` equal shares of the tile's K
-  // chunks (t0, c0 and nch below are the share's); with nparts > 1 it stores its partial tile at workspace tile ws_unit + part, and the
-  // ticket counter cnt_idx picks the CTA that sums the tile's partials
+  // chunks (t0, c0 and nch below are the share's); with nparts > 1 it stores its partial tile at
+  // workspace tile ws_unit + part, and the ticket counter cnt_idx picks the CTA that sums the tile's
+  // partials
   int32_t part, nparts, ws_unit, cnt_idx;
   // the share's first chunk (chunk c0 of term t0) and its number of chunks
   int32_t c0, nch;
@@ -77,9 +78,10 @@ struct Tile {
 static_assert(sizeof(Tile) == 64, "Tile layout");
 
 // K chunks of a term: the fewest chunks of at most 16 * kMaxKSteps, of equal length in multiples of
-// 16.  Digit products sum exactly up to K = 113 (kernels_f64.cu); H_AC applies with chunks of at most
-// 96, 80, 64 and 48 took 49.6, 45.3, 45.6 and 49.6 us (Hubbard D = 1024) and 18.5, 18.5, 18.5 and
-// 19.5 us (XXZ D = 512): longer ones cost shared memory for digits, shorter ones more FP64 work.
+// 16.  Digit products sum exactly up to K = 127 (kernels_f64.cu); with chunks of at most 80, 64 and 48 the
+// H_AC apply takes 47.4, 47.4 and 54.3 us (Hubbard D = 1024) and 18.8, 18.2 and 19.1 us (XXZ D = 512), the
+// transfer matrix 35.5, 37.7 and 45.7 us (XXZ D = 512): longer ones cost registers and shared memory for
+// digits, shorter ones more FP64 work.
 constexpr int kMaxKSteps = 5;
 inline int chunk_len(int k) {
   const int n = k > 0 ? (k + 16 * kMaxKSteps - 1) / (16 * kMaxKSteps) : 1;

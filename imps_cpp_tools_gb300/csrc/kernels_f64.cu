@@ -6,24 +6,35 @@
 // FP16 digits (the error-free splitting of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59 (2012)
 // 95, in the fixed-point form used on tensor cores by Mukunoki, Ozaki, Ogita and Imamura, ISC 2020):
 //   * a row of op(A), or a column of op(B), inside one K chunk of one term is scaled by a power of
-//     two to magnitude < 1 and rounded to 56 fractional bits (its largest entries keep all 53 bits
-//     of theirs), then written as 7 balanced base-256 digits d_0..d_6, |d_0| <= 256, |d_i| <= 128;
-//   * digit products of one level l = i + j <= 6 (28 of the 49 pairs) are summed in FP32 by mma.sync
-//     m16n8k16.  Every partial sum is an integer of at most 9 * 2^14 * 80 < 2^24, so the sums are
-//     exact in any order; the dropped levels and the rounding of the operands are below 2^-54 of the
-//     product of the two scales;
-//   * per output and chunk the seven level sums are combined in integers, converted to FP64 and added
-//     by one fma: one FP64 instruction where the direct form needs one per k.
-// Relative error of the H_AC apply (2-norm, against a double-double reference): 1.0e-16 to 1.3e-16 over
-// XXZ D = 32 to 1024 and Hubbard D = 64 to 1024, where the direct form had 1.5e-16 (D = 32) to 5.3e-16
-// (XXZ D = 1024); at XXZ D = 512 1.1e-16 after 4.2e-16, at Hubbard D = 1024 1.2e-16 after 4.7e-16.
+//     two to magnitude < 127 / 128 and cut off at 63 fractional bits (entries down to 2^-10 of the
+//     largest keep all 53 bits of theirs), then written as 8 balanced base-256 digits, |d_i| <= 128;
+//   * digit products of one level l = i + j <= 7 (36 of the 64 pairs) are summed in FP32 by mma.sync
+//     m16n8k16.  Every partial sum is an integer of at most 8 * 2^14 * 80 < 2^24, so the sums are
+//     exact in any order; the dropped levels and the cut operands are below 2^-60.5 of the product of
+//     the two scales for each k;
+//   * per output and chunk the eight level sums are combined in integers, converted to FP64 and added
+//     by one fma: one FP64 instruction where the direct form needs one per k;
+//   * that error is relative to the largest entries of the row and the column, an FP64 sum's to
+//     S = sum_k |a_ik| |b_kj|, which is far smaller where they are graded oppositely along k.  So
+//     one more product sums |d_0| |d_0|: from kTrusted = 256 on, S is above 2^-7.2 of the scales (the
+//     first digits may overstate it 2.3 times), and the error below K 2^-53 S, the bound of K FP64
+//     multiply-adds.  An output below it, other than one of a row or column of zeros, is computed by
+//     plain FP64 multiply-adds.  None are at Gaussian operands; at a converged VUMPS state of XXZ
+//     D = 512 up to 0.3% of those of an environment's products are.
+// Relative error of the H_AC apply (2-norm, against a double-double reference): 0.9e-16 to 1.1e-16 over
+// XXZ D = 32 to 1024 and Hubbard D = 64 to 1024, where the direct form had 1.4e-16 (D = 64) to 5.3e-16
+// (XXZ D = 1024); at XXZ D = 512 0.9e-16 after 4.1e-16, at Hubbard D = 1024 1.0e-16 after 4.7e-16.
+// Seven digits (28 products) without that test took 16.9 us instead of 18.8 (XXZ D = 512), but lost what is
+// small: a thick restart's rotation had 1.1e-15 in the lowest Ritz vector where the direct form has 3e-16
+// (now 2e-17), and VUMPS sweeps from starts 1e-16 apart had energies 1e-11 apart after one sweep (now
+// 1e-14, as with the direct form).
 // A chunk with an entry that is not finite, or with a row or column whose largest magnitude is outside
 // 2^-423 .. 2^477 (where the scaled sums could leave the FP64 range), is computed by plain FP64
 // fused multiply-adds, so infinities, NaN and extreme scales keep their FP64 results; so is one whose
 // op(A) has at most one entry per row, or op(B) per column (copies by an identity stay exact).
 //
 // mma.sync rather than tcgen05: the operands are split in registers on the fly (no operand packs that
-// could go stale, no extra pass over memory), blocks are ragged with edges from 1 to 82, and the seven
+// could go stale, no extra pass over memory), blocks are ragged with edges from 1 to 82, and the eight
 // level sums of a 16 x 8 sub-tile fit a warp's registers, where a 128-row instruction would compute
 // mostly padding.  What bounds it (XXZ D = 512 H_AC, ncu): integer pipe 29%, tensor pipe 16%, FP64 pipe
 // 13% busy, i.e. the latency of the chain load - split - multiply - combine of one to three chunks per
@@ -37,11 +48,11 @@
 // writes the tile.  Deterministic for a given plan; the first write also performs the reference's
 // memset of `out`, VUMPS_helpers.hpp:69.
 //
-// H_AC apply, direct FP64 form -> this one: XXZ D = 64 23.2 -> 6.8 us, XXZ D = 512 59.4 -> 16.9 us,
-// Hubbard D = 1024 163.7 -> 42.2 us; four-stage transfer matrix at XXZ D = 512 73.8 -> 32.3 us.
-// Dividing the work between warps that split and warps that multiply, in a persistent CTA per SM, gave
-// 15.5, 38.4 and 29.9 us, but 56.5 for 50.7 us on the projected transfer matrix at Hubbard D = 1024: the
-// SM's issue slots (some 10,000 warp instructions a chunk) are the limit, not the overlap.
+// H_AC apply, direct FP64 form -> this one: XXZ D = 64 23.2 -> 7.0 us, XXZ D = 512 59.4 -> 18.8 us,
+// Hubbard D = 1024 163.7 -> 47.4 us; four-stage transfer matrix at XXZ D = 512 73.8 -> 35.4 us.
+// Dividing the work between warps that split and warps that multiply, in a persistent CTA per SM, gained 8
+// to 9% on the H_AC applies (with seven digits), but lost 11% on the projected transfer matrix at Hubbard
+// D = 1024: the SM's issue slots (some 10,000 warp instructions a chunk) are the limit, not the overlap.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -55,8 +66,9 @@ using imps::Tile;
 
 namespace {
 
-constexpr int NS = 7;     // digits per operand
+constexpr int NS = 8;     // digits per operand
 constexpr int kLowExp = 600, kHighExp = 1500;  // biased exponents of rows the split form takes
+constexpr float kTrusted = 256.f;  // least sum of |first digit| |first digit| of an output that the digits give
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -78,38 +90,32 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], u
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// x / 2^(E - 1022) as a fixed-point integer with 56 fractional bits (rounded), plus a bias that makes
-// every base-256 digit non-negative: byte i < 6 holds digit d_{6-i} + 128, the top 16 bits d_0 + 512.
+// x / 2^(E - 1022) as a fixed-point integer with 63 fractional bits (cut off towards zero), |x| below 127 / 128 of
+// that scale, plus a bias that makes every base-256 digit non-negative: byte i holds digit d_{7-i} + 128.
 __device__ __forceinline__ uint64_t fixed_digits(double x, int E) {
   const uint32_t lo = (uint32_t)__double2loint(x);
   const int32_t hi = __double2hiint(x);
   const int e = (int)((2u * (uint32_t)hi) >> 21);
-  // the significand in bits 62..10, with the sign (as ones' complement: one unit in bit 0); an entry
-  // below the normal range is far below the row's scale, as is zero
+  // the significand in bits 62..10, with the sign as ones' complement; an entry below the normal range is
+  // far below the row's scale, as is zero
   const uint32_t sg = (uint32_t)(hi >> 31);
   const uint32_t th = __funnelshift_l(lo, ((uint32_t)hi & 0x000fffffu) | 0x00100000u, 10) ^ sg, tl = (lo << 10) ^ sg;
   const int64_t s = (int64_t)(((uint64_t)th << 32) | tl);
-  const int sh = min(E - e + 6, 63);
-  return (uint64_t)(((s >> sh) + (int64_t)(2 * 0x0200808080808080ull + 1)) >> 1);
+  return (uint64_t)(s >> min(E - e, 63)) + (0x8080808080808080ull + (sg & 1u));
 }
 
-// the seven digits of two entries (k, k + 1) as packed FP16: 1024 + u, less 1024 and the bias
+// the eight digits of two entries (k, k + 1) as packed FP16: 1024 + u, less 1024 and the bias
 __device__ __forceinline__ void digit_pairs(uint64_t x, uint64_t y, uint32_t (&d)[NS]) {
   const uint32_t xl = (uint32_t)x, yl = (uint32_t)y, xh = (uint32_t)(x >> 32), yh = (uint32_t)(y >> 32);
   const uint32_t m = 0x64646464u;
-  const uint32_t p0 = __byte_perm(xl, yl, 0x5140), p1 = __byte_perm(xl, yl, 0x7362), p2 = __byte_perm(xh, yh, 0x5140);
-  d[6] = __byte_perm(p0, m, 0x4140);
-  d[5] = __byte_perm(p0, m, 0x4342);
-  d[4] = __byte_perm(p1, m, 0x4140);
-  d[3] = __byte_perm(p1, m, 0x4342);
-  d[2] = __byte_perm(p2, m, 0x4140);
-  d[1] = __byte_perm(p2, m, 0x4342);
-  d[0] = __byte_perm(xh, yh, 0x7632) | 0x64006400u;
+  const uint32_t p[4] = {__byte_perm(xl, yl, 0x5140), __byte_perm(xl, yl, 0x7362), __byte_perm(xh, yh, 0x5140),
+                         __byte_perm(xh, yh, 0x7362)};
 #pragma unroll
   for (int i = 0; i < NS; ++i) {
-    const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&d[i]),
-                              __half2half2(__ushort_as_half(i == 0 ? 0x6600 : 0x6480)));  // 1536 or 1152
-    d[i] = *reinterpret_cast<const uint32_t*>(&h);
+    d[NS - 1 - i] = __byte_perm(p[i / 2], m, i & 1 ? 0x4342 : 0x4140);
+    const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&d[NS - 1 - i]),
+                              __half2half2(__ushort_as_half(0x6480)));  // 1152
+    d[NS - 1 - i] = *reinterpret_cast<const uint32_t*>(&h);
   }
 }
 
@@ -141,7 +147,7 @@ enum : int {
 };
 
 // digits of the held entries into the planes dg[NS][TILE][RS bytes] and the rows' biased exponents into
-// ex[TILE] (1023 for a row of zeros); returns the row's flags
+// ex[TILE] (0 for a row of zeros); returns the row's flags
 template <int KI, int TILE>
 __device__ __forceinline__ int store_digits(const double (&v)[4 * KI], int steps, int* ex, unsigned char* dg, int w,
                                             int lane) {
@@ -164,8 +170,10 @@ __device__ __forceinline__ int store_digits(const double (&v)[4 * KI], int steps
     sum += __shfl_xor_sync(0xffffffffu, sum, o);
     any |= __shfl_xor_sync(0xffffffffu, any, o);
   }
-  const int E = any == 0 ? 1023 : (int)(m >> 21), r = 8 * w + (lane & 7);
-  if (lane < 8) ex[r] = E;
+  // the next power of two, or the one after it for a largest entry above 127 / 128 of it, whose first digit
+  // could be 128
+  const int E = any == 0 ? 1023 : (int)((m + (1u << 15)) >> 21), r = 8 * w + (lane & 7);
+  if (lane < 8) ex[r] = any == 0 ? 0 : E;
   unsigned char* d = dg + r * RS + 4 * (lane >> 3);
 #pragma unroll
   for (int i = 0; i < 2 * KI; ++i)
@@ -175,17 +183,77 @@ __device__ __forceinline__ int store_digits(const double (&v)[4 * KI], int steps
 #pragma unroll
       for (int s = 0; s < NS; ++s) *reinterpret_cast<uint32_t*>(d + 16 * i + s * PL) = dp[s];
     }
-  return (E < kLowExp || E > kHighExp ? kUnsplittable : 0) | (sum > (m >> 21) ? kSeveral : any != 0 ? kOne : 0);
+  const int top = (int)(m >> 21);
+  return (any != 0 && (top < kLowExp || top > kHighExp) ? kUnsplittable : 0) |
+         (sum > (m >> 21) ? kSeveral : any != 0 ? kOne : 0);
 }
 
-// the level sums of a warp's m16 x n8 sub-tile over the chunk's K steps (16 x 16 tiles: every other
-// one), combined and added to facc
+// a chunk's operands: entry (r, k) of op(A) (rows m) or op(B)^T (rows n) at r * sr + k * sk
+struct Chunk {
+  const double *a, *b;
+  int asr, ask, bsr, bsk, len;
+  double alpha;
+};
+
+// a warp's k of a chunk: all of them, in a 16 x 16 tile those of every other K step
+template <int TILE>
+__device__ __forceinline__ int nth_k(int i, int ks0) { return TILE == 16 ? 32 * (i >> 4) + 16 * ks0 + (i & 15) : i; }
+template <int TILE>
+__device__ __forceinline__ int num_k(int len, int ks0) {
+  return TILE == 16 ? (len >> 5) * 16 + min(16, max(0, (len & 31) - 16 * ks0)) : len;
+}
+
+// a warp's m16 x n8 sub-tile of a chunk in plain FP64, added to facc; rows and columns past the tile's edge
+// repeat its last ones and are not written
+template <int TILE>
+__device__ __forceinline__ void plain_products(const Chunk& ch, int mt, int nt, int m0, int n0, int ks0, int lane,
+                                               double (&facc)[4]) {
+  const double* a[2];
+  const double* b[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    a[h] = ch.a + (int64_t)min(m0 + (lane >> 2) + 8 * h, mt - 1) * ch.asr;
+    b[h] = ch.b + (int64_t)min(n0 + 2 * (lane & 3) + h, nt - 1) * ch.bsr;
+  }
+  const int n = num_k<TILE>(ch.len, ks0);
+#pragma unroll 2
+  for (int i = 0; i < n; ++i) {
+    const int64_t k = nth_k<TILE>(i, ks0);
+    double x[2] = {a[0][k * ch.ask], a[1][k * ch.ask]};
+    const double y[2] = {b[0][k * ch.bsk], b[1][k * ch.bsk]};
+    if (ch.alpha != 1.0) {
+      x[0] *= ch.alpha;
+      x[1] *= ch.alpha;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) facc[q] = fma(x[q >> 1], y[q & 1], facc[q]);
+  }
+}
+
+// one output of a chunk in plain FP64 by a warp, in every lane
+template <int TILE>
+__device__ __noinline__ double plain_output(const double* a, int ask, const double* b, int bsk, int len, double alpha,
+                                            int ks0, int lane) {
+  const int n = num_k<TILE>(len, ks0);
+  double s = 0.0;
+  for (int i = lane; i < n; i += 32) {
+    const int64_t k = nth_k<TILE>(i, ks0);
+    s = fma(alpha * a[k * ask], b[k * bsk], s);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+// the products of a warp's m16 x n8 sub-tile over the chunk's K steps (16 x 16 tiles: every other one), added
+// to facc
 template <int KI, int TILE>
 __device__ __forceinline__ void chunk_products(const unsigned char* da, const unsigned char* db, const int* ea,
-                                               const int* eb, int m0, int n0, int ks0, int steps, double alpha, int lane,
-                                               double (&facc)[4]) {
+                                               const int* eb, const Chunk& ch, int mt, int nt, int m0, int n0, int ks0,
+                                               int lane, double (&facc)[4]) {
   constexpr int RS = 32 * KI + 16, PL = TILE * RS;
-  float acc[NS][4];
+  const int steps = (ch.len + 15) >> 4;
+  float acc[NS][4], mag[4] = {0.f, 0.f, 0.f, 0.f};  // level sums; sum of |first digit| |first digit|
 #pragma unroll
   for (int l = 0; l < NS; ++l)
 #pragma unroll
@@ -203,22 +271,51 @@ __device__ __forceinline__ void chunk_products(const unsigned char* da, const un
       ldsm4(a, aa + i * PL + ks * 32);
 #pragma unroll
       for (int s = 0; s + i < NS; ++s) mma_f16(acc[i + s], a, b[s][0], b[s][1]);
+      if (i == 0) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) a[q] &= 0x7fff7fffu;
+        mma_f16(mag, a, b[0][0] & 0x7fff7fffu, b[0][1] & 0x7fff7fffu);
+      }
     }
   }
-  const int g = lane >> 2, t = lane & 3;
+  double w[4];
+  bool bad[4];
+  int nbad = 0;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     int L[NS];
 #pragma unroll
     for (int l = 0; l < NS; ++l) L[l] = __float2int_rn(acc[l][q]);
-    // sum of L[l] 2^(-8 l), in units of 2^-40: 63 bits and a sign; the lowest 8 bits are rounded off
-    const int64_t hi = ((int64_t)L[0] << 24) + ((int64_t)L[1] << 16) + ((int64_t)L[2] << 8) + L[3];
-    const int64_t lo = ((int64_t)L[4] << 16) + ((int64_t)L[5] << 8) + L[6];
-    const double v = (double)((hi << 16) + ((lo + 128) >> 8));
-    // times 2^(ea + eb - 2044 - 56), by the exponent field (in range: see kLowExp, kHighExp)
-    const int s = ea[m0 + g + (q & 2 ? 8 : 0)] + eb[n0 + 2 * t + (q & 1)] - 2100;
-    const double w = v == 0.0 ? 0.0 : __hiloint2double(__double2hiint(v) + (s << 20), __double2loint(v));
-    facc[q] = fma(alpha, w, facc[q]);
+    // sum of L[l] 2^(-8 l) in units of 2^-56, as hi 2^32 + lo, and its highest 64 bits as w 2^(32 - z)
+    int64_t hi = ((int64_t)((L[0] << 8) + L[1]) << 16) + ((L[2] << 8) + L[3]);
+    const int64_t lo = ((int64_t)((L[4] << 8) + L[5]) << 16) + ((int64_t)L[6] << 8) + L[7];
+    hi += lo >> 32;
+    const int z = min(__clzll(hi ^ (hi >> 63)) - 1, 32);
+    const double v = (double)((hi << z) + (int64_t)(((uint64_t)(uint32_t)lo << z) >> 32));
+    // times 2^(ea + eb - 2044 - 70 + 32 - z), by the exponent field (in range: see kLowExp, kHighExp)
+    const int m = m0 + (lane >> 2) + (q & 2 ? 8 : 0), n = n0 + 2 * (lane & 3) + (q & 1);
+    const int sa = ea[m], sb = eb[n], s = sa + sb - 2082 - z;
+    w[q] = v == 0.0 ? 0.0 : __hiloint2double(__double2hiint(v) + (s << 20), __double2loint(v));
+    bad[q] = mag[q] < kTrusted && sa != 0 && sb != 0 && m < mt && n < nt;
+    nbad += __popc(__ballot_sync(0xffffffffu, bad[q]));
+  }
+  // outputs that the digits do not hold well enough, one by one or all at once, whichever is shorter (some 1,000
+  // cycles each, or 400 for every k)
+  if (5 * nbad > 2 * num_k<TILE>(ch.len, ks0)) {
+    plain_products<TILE>(ch, mt, nt, m0, n0, ks0, lane, facc);
+    return;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    if (!bad[q]) facc[q] = fma(ch.alpha, w[q], facc[q]);
+    if (nbad > 0)
+      for (uint32_t todo = __ballot_sync(0xffffffffu, bad[q]); todo; todo &= todo - 1) {
+        const int l = __ffs(todo) - 1;
+        const double* a = ch.a + (int64_t)(m0 + (l >> 2) + (q & 2 ? 8 : 0)) * ch.asr;
+        const double* b = ch.b + (int64_t)(n0 + 2 * (l & 3) + (q & 1)) * ch.bsr;
+        const double x = plain_output<TILE>(a, ch.ask, b, ch.bsk, ch.len, ch.alpha, ks0, lane);
+        if (lane == l) facc[q] += x;
+      }
   }
 }
 
@@ -249,11 +346,7 @@ grouped_gemm_f64_kernel(const Tile* __restrict__ tiles, const Term* __restrict__
   const bool mine = n0 < tl.nt, splits = 8 * w4 < (side ? tl.nt : tl.mt);
   double facc[4] = {0.0, 0.0, 0.0, 0.0};
 
-  struct Chunk {
-    const double *a, *b;
-    int asr, ask, bsr, bsk, len;  // strides along the rows (m, n) and along k
-    double alpha;
-  } cur{}, prev{};
+  Chunk cur{}, prev{};
   double v[4 * KI];
   bool direct = false;  // the split chunk is to be computed by plain FP64
   int t = tl.t0, c = tl.c0;
@@ -282,26 +375,11 @@ grouped_gemm_f64_kernel(const Tile* __restrict__ tiles, const Term* __restrict__
                          side ? tl.nt : tl.mt, cur.len, w4, lane);
     }
     if (it > 0) {
-      const int steps = (prev.len + 15) >> 4;
-      if (mine && !direct) {
-        if (ks0 < steps)
-          chunk_products<KI, TILE>(digits, digits + NS * PL, ex, ex + TILE, m0, n0, ks0, steps, prev.alpha, lane, facc);
-      } else if (mine && ks0 == 0) {
-        // plain FP64; rows and columns past the tile's edge repeat its last ones and are not written
-        const double* a[2];
-        const double* b[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          a[h] = prev.a + (int64_t)min(m0 + (lane >> 2) + 8 * h, tl.mt - 1) * prev.asr;
-          b[h] = prev.b + (int64_t)min(n0 + 2 * (lane & 3) + h, tl.nt - 1) * prev.bsr;
-        }
-#pragma unroll 2
-        for (int k = 0; k < prev.len; ++k) {
-          const double x[2] = {prev.alpha * a[0][(int64_t)k * prev.ask], prev.alpha * a[1][(int64_t)k * prev.ask]};
-          const double y[2] = {b[0][(int64_t)k * prev.bsk], b[1][(int64_t)k * prev.bsk]};
-#pragma unroll
-          for (int q = 0; q < 4; ++q) facc[q] = fma(x[q >> 1], y[q & 1], facc[q]);
-        }
+      if (mine && 16 * ks0 < prev.len) {
+        if (direct)
+          plain_products<TILE>(prev, tl.mt, tl.nt, m0, n0, ks0, lane, facc);
+        else
+          chunk_products<KI, TILE>(digits, digits + NS * PL, ex, ex + TILE, prev, tl.mt, tl.nt, m0, n0, ks0, lane, facc);
       }
       if (it == tl.nch) break;
       __syncthreads();  // the previous chunk's digits are no longer read
@@ -315,8 +393,7 @@ grouped_gemm_f64_kernel(const Tile* __restrict__ tiles, const Term* __restrict__
     }
     __syncthreads();
     // An operand whose rows (columns) hold one entry each at most selects and scales the other's
-    // entries: plain FP64 gives each its own 53 bits, where the split form would round it to the
-    // scale of its row.
+    // entries: plain FP64 gives each product its own 53 bits.
     const int f = flags[it & 1];
     direct = (f & kUnsplittable) || (f & (kOne | kSeveral)) == kOne || (f & (kOneB | kSeveralB)) == kOneB;
     if (threadIdx.x == 0) flags[(it + 1) & 1] = 0;  // written again after the next barrier
@@ -417,14 +494,15 @@ int imps_launch_grouped_f64(const void* d_tiles, int ntiles, const void* d_terms
 int imps_launch_grouped_f64(const void* d_tiles, int ntiles, const void* d_terms, const imps_planes& planes, int tile,
                             int ksteps, int splits, double* ws, int* cnt, void* stream, bool after_tables) {
   if (ntiles <= 0) return IMPS_OK;
-  if (planes.n < 1 || planes.n > 2 || splits < 1 || (splits > 1 && (!ws || !cnt)) || (tile != 16 && tile != 32)) return IMPS_ERR_BAD_ARG;
+  if (planes.n < 1 || planes.n > 2 || splits < 1 || (splits > 1 && (!ws || !cnt)) || (tile != 16 && tile != 32))
+    return IMPS_ERR_BAD_ARG;
   KernelFn fn = tile == 16 ? kernel_of<16>(ksteps) : kernel_of<32>(ksteps);
   if (!fn) return IMPS_ERR_BAD_ARG;
   imps::count_launch();
   const int smem = tile == 16 ? smem_bytes<16>(ksteps) : smem_bytes<32>(ksteps);
   if (after_tables) {
-    fn<<<dim3(ntiles, planes.n), dim3(tile * 8), smem, (cudaStream_t)stream>>>((const Tile*)d_tiles, (const Term*)d_terms, planes,
-                                                                               ws, cnt);
+    fn<<<dim3(ntiles, planes.n), dim3(tile * 8), smem, (cudaStream_t)stream>>>((const Tile*)d_tiles,
+                                                                               (const Term*)d_terms, planes, ws, cnt);
     return cudaGetLastError() == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
   }
   const cudaError_t e = imps::launch_overlapped(fn, dim3(ntiles, planes.n), dim3(tile * 8), smem, (cudaStream_t)stream,
