@@ -901,7 +901,8 @@ __device__ __forceinline__ bool rotation(double& al, double& be, double ga, doub
 // has |<b_i, b_j>| <= tol |b_i| |b_j|: the sweep rotated nothing, or so little that it left no more.  (A pair
 // that the sweep has made orthogonal gets products back from later rotations of either column with a third:
 // at most N of the size mr max(mr, mt), for the largest ratio |<b_i, b_j>| / |b_i| |b_j| and tangent that
-// the sweep met; so `rest` = tol / N does.)  nrm_g: squared column norms (scratch).  An FP64 instruction takes 64 cycles of its
+// the sweep met; so `rest` = tol / N does.  And the FP32 tangent, within 2^-21 of the right one, leaves
+// a pair up to 2^-21 of its ratio, more than tol for narrow sectors.)  nrm_g: squared column norms (scratch).  An FP64 instruction takes 64 cycles of its
 // scheduler however many lanes it serves and a round of N = 68 has 5 pairs, so a pair has 16 lanes: warps
 // 0-3 take products, parameters and B, the others V, one turn behind.
 // G lanes per pair with R rows each (N <= G R; loops of fixed length: a branch per step cost 20 cycles each).
@@ -1065,7 +1066,7 @@ __device__ int cluster_sweeps(T* B, T* V, T* nrm_g, int N, T tol, float rest, in
     }
     cluster_sync();  // every flag has been read before it is reset
     mr = __int_as_float(ir);
-    if (mr * fmaxf(mr, __int_as_float(it)) <= rest) return sweep + 1;
+    if (mr * fmaxf(mr, __int_as_float(it)) <= rest && mr * 0x1p-21f <= (float)tol) return sweep + 1;
   }
   return max_sweeps + 1;
 }
@@ -1309,8 +1310,11 @@ svd_cluster_kernel(const imps::SvdSets sets, int smem_doubles, int max_sweeps, i
   // ---- B = X V in V's place, and the FP64 sweeps
   product(U, false, vc, yc, 0.0, 1.0, false);
   publish(Vo, yc);
-  const double tol = (double)N * 2.220446049250313e-16;
-  const int sw = cluster_sweeps<double>(Vo, W, S, N, tol, 2e-16f, max_sweeps, buf, sweep_s, rank);
+  // N eps a pair up to N = 16, as the one-CTA form; wider sectors 16 eps, above the rounding of a rotation and a
+  // product of 16 lanes (12 eps at most), so that V is as orthogonal as after one-CTA sweeps that end only when
+  // they find nothing to rotate: |V^T V - 1| at N = 100 4e-13 with N eps, 6e-14 so, in the same time
+  const double tol = fmin((double)N, fmax(16.0, 0.125 * N)) * 2.220446049250313e-16;
+  const int sw = cluster_sweeps<double>(Vo, W, S, N, tol, (float)(tol / N), max_sweeps, buf, sweep_s, rank);
   if (threadIdx.x == 0 && rank == 0 && sw > max_sweeps && status) atomicExch(status, 1);
 
   // ---- singular values, descending (ties by index; what is not a number last), in every CTA
