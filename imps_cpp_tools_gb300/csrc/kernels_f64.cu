@@ -203,31 +203,39 @@ __device__ __forceinline__ int num_k(int len, int ks0) {
   return TILE == 16 ? (len >> 5) * 16 + min(16, max(0, (len & 31) - 16 * ks0)) : len;
 }
 
-// a warp's m16 x n8 sub-tile of a chunk in plain FP64, added to facc; rows and columns past the tile's edge
-// repeat its last ones and are not written
-template <int TILE>
-__device__ __forceinline__ void plain_products(const Chunk& ch, int mt, int nt, int m0, int n0, int ks0, int lane,
-                                               double (&facc)[4]) {
-  const double* a[2];
-  const double* b[2];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    a[h] = ch.a + (int64_t)min(m0 + (lane >> 2) + 8 * h, mt - 1) * ch.asr;
-    b[h] = ch.b + (int64_t)min(n0 + 2 * (lane & 3) + h, nt - 1) * ch.bsr;
-  }
+template <int TILE, bool SCALED>
+__device__ __forceinline__ void plain_sums(const Chunk& ch, const double* const (&a)[2], const double* const (&b)[2],
+                                           int ks0, double (&facc)[4]) {
   const int n = num_k<TILE>(ch.len, ks0);
 #pragma unroll 2
   for (int i = 0; i < n; ++i) {
     const int64_t k = nth_k<TILE>(i, ks0);
     double x[2] = {a[0][k * ch.ask], a[1][k * ch.ask]};
     const double y[2] = {b[0][k * ch.bsk], b[1][k * ch.bsk]};
-    if (ch.alpha != 1.0) {
+    if (SCALED) {
       x[0] *= ch.alpha;
       x[1] *= ch.alpha;
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) facc[q] = fma(x[q >> 1], y[q & 1], facc[q]);
   }
+}
+
+// a warp's m16 x n8 sub-tile of a chunk in plain FP64, added to facc; rows and columns past the tile's edge
+// repeat its last ones and are not written
+template <int TILE>
+__device__ __forceinline__ void plain_products(const Chunk& ch, int mt, int nt, int m0, int n0, int ks0, int lane,
+                                               double (&facc)[4]) {
+  const double *a[2], *b[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    a[h] = ch.a + (int64_t)min(m0 + (lane >> 2) + 8 * h, mt - 1) * ch.asr;
+    b[h] = ch.b + (int64_t)min(n0 + 2 * (lane & 3) + h, nt - 1) * ch.bsr;
+  }
+  // two loops: FP64 multiplications under a predicate that is off take their time all the same (one-site
+  // transfer matrix of the identity, XXZ D = 512: 43 us, 32 so)
+  if (ch.alpha == 1.0) plain_sums<TILE, false>(ch, a, b, ks0, facc);
+  else plain_sums<TILE, true>(ch, a, b, ks0, facc);
 }
 
 // one output of a chunk in plain FP64 by a warp, in every lane
