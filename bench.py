@@ -55,7 +55,7 @@ L2_FLUSH_BYTES = 512 << 20
 # (profiles/tc_gemm_hac_xxz_d512.md: tc_gemm 2.73 MB, and 0.40 MB of the pack's input;
 # profiles/grouped_gemm_f64_hac_xxz_d512.md, autotuned shape 32x32 with 4 shares: 2.39 MB)
 NCU_TRAFFIC_BYTES = {"bf16x6": 3.13e6, "fp64": 2.39e6}
-FP16_DIGIT_PRODUCTS = 28
+FP16_DIGIT_PRODUCTS = 37  # 36 of the digits, one of the first digits' magnitudes
 # tolerances of the timed sweeps: the eigensolver tolerance of the configuration (1e-12); GMRES
 # 1e-8, because the environment systems of these states do not reach 1e-12 in floating point:
 # measured at XXZ D=512 from the warmed state, the relative residual of the left-environment
@@ -527,7 +527,7 @@ def run_vumps(args):
                 "frac": achieved / bf16_peak, "traffic": NCU_TRAFFIC_BYTES["fp64"],
                 "peak_source": "MEASURED_PEAKS.json bf16_tflops (burst), of measured; mma.sync, which this kernel "
                                "issues, reaches about a third of it on this GPU",
-                "kernel": "grouped_gemm_f64 (H_AC apply; 28 FP16 digit products per FP64 product; the dominant kernel "
+                "kernel": "grouped_gemm_f64 (H_AC apply; 37 FP16 digit products per FP64 product; the dominant kernel "
                           "of the timed sweeps)",
                 "fp64_equivalent": {"achieved": flops / t_hac64 / 1e12, "peak": fp64_peak,
                                     "frac": flops / t_hac64 / 1e12 / fp64_peak, "peak_source": fp64_src},

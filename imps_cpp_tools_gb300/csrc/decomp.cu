@@ -3,7 +3,8 @@
 // The reference stacks, per charge sector, the blocks of A_s into one dense matrix
 // (MPSBlockMat::GetDenseMat, MPSBlockMat.hpp:468-526 with GetSingleSecData :636-719) and
 // runs LAPACK on it: qr_econ + sign fix (qr_pos, helpers.hpp:181-195) or svd_econ
-// (MPSBlockUtilities.hpp:78-244, BlockObj.hpp:2422-2541).  Here every sector is one CTA:
+// (MPSBlockUtilities.hpp:78-244, BlockObj.hpp:2422-2541).  Here a sector is the work of a cluster of
+// eight CTAs (QR, SVD; one CTA where a sector of the call does not fit a cluster) or of one CTA (null space):
 //  * gather: blocks -> packed column-major dense matrices (transposed for dir = r, so that
 //    every matrix is handled as "tall": M = stacked dimension, N = sector dimension);
 //  * Householder QR with explicit Q and diag(R) >= 0;
@@ -331,7 +332,8 @@ qr_cluster_kernel(const imps::DenseMat* __restrict__ mats, const double* __restr
     if (k + 1 < N) cluster_arrive();
     if (next) __syncthreads();  // the FP64 pipe is the maker's until reflector k + 1 is made
     if (tau != 0.0)
-      for (int jl = first + (next ? 1 : 0) + warp; jl < mine; jl += QT / 32) reflect(cols + (size_t)jl * M, v, tau, M, k, lane);
+      for (int jl = first + (next ? 1 : 0) + warp; jl < mine; jl += QT / 32)
+        reflect(cols + (size_t)jl * M, v, tau, M, k, lane);
   }
   __syncthreads();
   // R (N x N) with a non-negative diagonal: row i times sgn_i
@@ -360,7 +362,8 @@ qr_cluster_kernel(const imps::DenseMat* __restrict__ mats, const double* __restr
     for (int i = k + threadIdx.x; i < M; i += QT) v[i] = ld_cluster(src + i, k % QC);
     __syncthreads();
     if (tau != 0.0)
-      for (int jl = (k - rank + QC - 1) / QC + warp; jl < mine; jl += QT / 32) reflect(qc + jl * ldq, v, tau, M, k, lane);
+      for (int jl = (k - rank + QC - 1) / QC + warp; jl < mine; jl += QT / 32)
+        reflect(qc + jl * ldq, v, tau, M, k, lane);
   }
   cluster_arrive();
   if (q_shared) {
@@ -371,8 +374,8 @@ qr_cluster_kernel(const imps::DenseMat* __restrict__ mats, const double* __restr
   cluster_wait();  // no CTA leaves while another may still read its columns
 }
 
-// The same for sectors whose columns do not fit a cluster's shared memory (M N over about 100,000):
-// one CTA, the matrix in global memory.
+// The same where a sector of the call does not fit a cluster's shared memory, (ceil(N / 8) + 2) M over 25,600
+// (M = N: 441 columns fit): one CTA, the matrix in global memory.
 // Householder QR of the M x N matrix A (in place, column-major, ld = M), K = min(M,N).
 // Outputs Q (M x K, ld M) and R (K x N, ld K) with diag(R) >= 0.
 __global__ void __launch_bounds__(DT) qr_kernel(const imps::DenseMat* __restrict__ mats,
@@ -447,9 +450,9 @@ __global__ void __launch_bounds__(DT) nullspace_kernel(const imps::DenseMat* __r
 }
 
 // One-sided Jacobi SVD of the M x N matrix held in U (in place, M >= N), in global memory (the
-// fallback where neither a cluster's nor one CTA's shared memory holds a sector): on exit U holds the left singular vectors (M x N), S the
-// singular values (descending), V the right singular vectors (N x N).  Round-robin pair
-// ordering; every warp rotates disjoint column pairs.
+// fallback where neither a cluster's nor one CTA's shared memory holds a sector): on exit U holds the
+// left singular vectors (M x N), S the singular values (descending), V the right singular vectors
+// (N x N).  Round-robin pair ordering; every warp rotates disjoint column pairs.
 __global__ void __launch_bounds__(DT) svd_kernel(const imps::DenseMat* __restrict__ mats,
                                                  double* __restrict__ U, double* __restrict__ S,
                                                  double* __restrict__ V, double* __restrict__ Wk,
@@ -785,18 +788,19 @@ __global__ void __launch_bounds__(JT) svd_pjac_kernel(const imps::SvdSets sets, 
 // the work of a sector spread over eight SMs:
 //   * Pivoted QR as in qr_cluster_kernel, columns staying in place: every CTA proposes the longest of its own
 //     remaining columns (its norm summed anew in each update) and the cluster takes the longest of the
-//     eight, so that a step needs one cluster barrier.
+//     eight, so that a step needs one cluster barrier (and two of the CTA's own).
 //   * Jacobi by blocks: the columns of B and V are 16 blocks in global memory (L2).  In each of 15 rounds a
 //     CTA loads two blocks, rotates the pairs between them (in the first round also those inside them) in
 //     shared memory, and stores them.  The tangent of a rotation is taken in FP32: it only decides how small
 //     the pair's product becomes.  Cosine and sine are FP64 with c^2 + s^2 = 1 to rounding.
 //   * V of the FP32 sweeps is made orthonormal by two Newton-Schulz steps V <- V (3 - V^T V) / 2 (error
-//     1e-6, 1e-12, rounding); the Cholesky factorisation of the one-CTA form is a serial chain.
+//     1e-6, 1e-12, rounding; at most 6e-4, 3e-7, 6e-14 if every rounding of eight sweeps of 95 rounds, 8e-7
+//     each, pulled the same way); the Cholesky factorisation of the one-CTA form is a serial chain.
 // What bounds it, for a 136 x 68 sector over four decades (one CTA -> cluster, us): the QR, 2,123 -> 345, a
-// chain of two barriers, a remote read, square root and division a step; the FP32 sweeps, 635 -> 433, the
+// chain of a cluster barrier, a remote read, square root and division a step; the FP32 sweeps, 635 -> 433, the
 // latency of a turn (920 cycles: 280 to load and multiply, 210 parameters, 130 to store); the FP64 sweeps,
 // 3,060 -> 458, FP64 instructions at 64 cycles a warp; the products, 300 -> 77; U, 795 -> 157.  The polar
-// step of XXZ D = 512 (both directions, 42 sectors): 6,690 -> 1,547 us.  20 equal sectors of N columns:
+// step of XXZ D = 512 (both directions, 42 sectors): 6,690 -> 1,610 us.  20 equal sectors of N columns:
 // N = 1 27 -> 27 us, 4 131 -> 81, 16 707 -> 377, 64 5,806 -> 1,259, 118 34,322 -> 4,231, so every sector that
 // fits comes here.
 constexpr int JB = 2 * QC;  // column blocks
@@ -902,9 +906,10 @@ __device__ __forceinline__ bool rotation(double& al, double& be, double ga, doub
 // that the sweep has made orthogonal gets products back from later rotations of either column with a third:
 // at most N of the size mr max(mr, mt), for the largest ratio |<b_i, b_j>| / |b_i| |b_j| and tangent that
 // the sweep met; so `rest` = tol / N does.  And the FP32 tangent, within 2^-21 of the right one, leaves
-// a pair up to 2^-21 of its ratio, more than tol for narrow sectors.)  nrm_g: squared column norms (scratch).  An FP64 instruction takes 64 cycles of its
-// scheduler however many lanes it serves and a round of N = 68 has 5 pairs, so a pair has 16 lanes: warps
-// 0-3 take products, parameters and B, the others V, one turn behind.
+// a pair up to 2^-21 of its ratio, more than tol for narrow sectors.)  nrm_g: squared column norms
+// (scratch).  An FP64 instruction takes 64 cycles of its scheduler however many lanes it serves and a round
+// of N = 68 has 5 pairs, so a pair has 16 lanes: warps 0-3 take products, parameters and B, the others V,
+// one turn behind.
 // G lanes per pair with R rows each (N <= G R; loops of fixed length: a branch per step cost 20 cycles each).
 // Returns the sweeps run, max_sweeps + 1 if the last one still rotated.
 struct SweepShared {
@@ -1495,7 +1500,8 @@ int dc_svd_sets(const SvdSets& sets, const std::vector<DenseMat>* const* mats, i
   if (maxN <= SVD_MAXN && least * sizeof(double) <= (size_t)SVD_SMEM) {
     imps::count_launch();
     // two CTAs per SM if U still fits, with the products in pieces
-    const size_t doubles = std::min(want, (size_t)(good * sizeof(double) <= SVD_SMEM2 ? SVD_SMEM2 : SVD_SMEM) / sizeof(double));
+    const size_t most = good * sizeof(double) <= SVD_SMEM2 ? SVD_SMEM2 : SVD_SMEM;
+    const size_t doubles = std::min(want, most / sizeof(double));
     svd_cluster_kernel<<<nmat * QC, QT, doubles * sizeof(double), st>>>(sets, (int)doubles, 30, status);
     return cudaGetLastError() == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
   }

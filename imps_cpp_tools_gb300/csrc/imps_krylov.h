@@ -45,7 +45,8 @@ int kr_cgs2_step(const KrylovWs& ws, const double* V, int64_t ldv, int nc, doubl
 int kr_cgs2_step_batch(double* partials, unsigned int* counters, int P, const double* V, int64_t sV, int64_t ldv,
                        int nc, double* w, int64_t sw, int64_t n, double* h, int64_t sh, double* h2, double* vnext,
                        int* flags, cudaStream_t st);
-// out (n x kk) = V (n x m) W (m x kk); scratch: kr_rotate_scratch(n, kk) bytes, 16-byte aligned, for the launch's tables
+// out (n x kk) = V (n x m) W (m x kk); scratch: kr_rotate_scratch(n, kk) bytes, 16-byte aligned, for the
+// launch's tables
 size_t kr_rotate_scratch(int64_t n, int kk);
 int kr_basis_rotate(const double* V, int64_t ldv, int m, const double* W, int kk, double* out,
                     int64_t ldo, int64_t n, void* scratch, cudaStream_t st);

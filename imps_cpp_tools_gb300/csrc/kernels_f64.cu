@@ -16,11 +16,13 @@
 //     by one fma: one FP64 instruction where the direct form needs one per k;
 //   * that error is relative to the largest entries of the row and the column, an FP64 sum's to
 //     S = sum_k |a_ik| |b_kj|, which is far smaller where they are graded oppositely along k.  So
-//     one more product sums |d_0| |d_0|: from kTrusted = 256 on, S is above 2^-7.2 of the scales (the
-//     first digits may overstate it 2.3 times), and the error below K 2^-53 S, the bound of K FP64
-//     multiply-adds.  An output below it, other than one of a row or column of zeros, is computed by
-//     plain FP64 multiply-adds.  None are at Gaussian operands; at a converged VUMPS state of XXZ
-//     D = 512 up to 0.3% of those of an environment's products are.
+//     one more product sums the magnitudes that the first two digits give, |256 d_0 + d_1| (an entry
+//     is within 0.502 of it: 80 products overstate S by at most 2.7e6 of the units of 2^-30).  From
+//     kTrusted on, S is thus above 2^-7.5 of the scales and the error below K 2^-53 S, the bound of
+//     K FP64 multiply-adds.  An output below it, other than one of a row or column of zeros, is computed
+//     by plain FP64 multiply-adds: none at Gaussian operands, below 1% in an environment's products at
+//     converged VUMPS states of XXZ D = 512.  (The first digit alone sees 0.3 to 6% of those as
+//     too small, an environment's entries off its diagonal being some 0.3% of those on it: H_AC 36 us.)
 // Relative error of the H_AC apply (2-norm, against a double-double reference): 0.9e-16 to 1.1e-16 over
 // XXZ D = 32 to 1024 and Hubbard D = 64 to 1024, where the direct form had 1.4e-16 (D = 64) to 5.3e-16
 // (XXZ D = 1024); at XXZ D = 512 0.9e-16 after 4.1e-16, at Hubbard D = 1024 1.0e-16 after 4.7e-16.
@@ -68,7 +70,7 @@ namespace {
 
 constexpr int NS = 8;     // digits per operand
 constexpr int kLowExp = 600, kHighExp = 1500;  // biased exponents of rows the split form takes
-constexpr float kTrusted = 256.f;  // least sum of |first digit| |first digit| of an output that the digits give
+constexpr float kTrusted = 9e6f;  // least magnitude sum, in units of 2^-30 of the scales, of an output that the digits give
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -80,7 +82,10 @@ __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
 }
 
 __device__ __forceinline__ void ldsm2(uint32_t (&r)[2], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr) : "memory");
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];"
+               : "=r"(r[0]), "=r"(r[1])
+               : "r"(addr)
+               : "memory");
 }
 
 __device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -238,30 +243,40 @@ __device__ __forceinline__ void plain_products(const Chunk& ch, int mt, int nt, 
   else plain_sums<TILE, true>(ch, a, b, ks0, facc);
 }
 
-// one output of a chunk in plain FP64 by a warp, in every lane
-template <int TILE>
-__device__ __noinline__ double plain_output(const double* a, int ask, const double* b, int bsk, int len, double alpha,
-                                            int ks0, int lane) {
-  const int n = num_k<TILE>(len, ks0);
+// one output of a chunk in plain FP64 by eight lanes (sub: the lane's number among them), in each of them
+template <int TILE, bool SCALED>
+__device__ __forceinline__ double plain_output(const Chunk& ch, int m, int n, int ks0, int sub) {
+  const double *a = ch.a + (int64_t)m * ch.asr, *b = ch.b + (int64_t)n * ch.bsr;
+  const int nk = num_k<TILE>(ch.len, ks0);
   double s = 0.0;
-  for (int i = lane; i < n; i += 32) {
+#pragma unroll 2
+  for (int i = sub; i < nk; i += 8) {
     const int64_t k = nth_k<TILE>(i, ks0);
-    s = fma(alpha * a[k * ask], b[k * bsk], s);
+    double x = a[k * ch.ask];
+    if (SCALED) x *= ch.alpha;
+    s = fma(x, b[k * ch.bsk], s);
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   return s;
 }
 
 // the products of a warp's m16 x n8 sub-tile over the chunk's K steps (16 x 16 tiles: every other one), added
 // to facc
+// |256 d_0 + d_1| of two entries, to FP16
+__device__ __forceinline__ uint32_t magnitude(uint32_t d0, uint32_t d1) {
+  const __half2 h = __hfma2(*reinterpret_cast<const __half2*>(&d0), __half2half2(__ushort_as_half(0x5c00)),  // 256
+                            *reinterpret_cast<const __half2*>(&d1));
+  return *reinterpret_cast<const uint32_t*>(&h) & 0x7fff7fffu;
+}
+
 template <int KI, int TILE>
 __device__ __forceinline__ void chunk_products(const unsigned char* da, const unsigned char* db, const int* ea,
-                                               const int* eb, const Chunk& ch, int mt, int nt, int m0, int n0, int ks0,
-                                               int lane, double (&facc)[4]) {
+                                               const int* eb, unsigned char* list, const Chunk& ch, int mt, int nt,
+                                               int m0, int n0, int ks0, int lane, double (&facc)[4]) {
   constexpr int RS = 32 * KI + 16, PL = TILE * RS;
   const int steps = (ch.len + 15) >> 4;
-  float acc[NS][4], mag[4] = {0.f, 0.f, 0.f, 0.f};  // level sums; sum of |first digit| |first digit|
+  float acc[NS][4], mag[4] = {0.f, 0.f, 0.f, 0.f};  // level sums; magnitude sums
 #pragma unroll
   for (int l = 0; l < NS; ++l)
 #pragma unroll
@@ -270,7 +285,7 @@ __device__ __forceinline__ void chunk_products(const unsigned char* da, const un
   const uint32_t aa = smem_addr(da) + (m0 + (lane & 15)) * RS + (lane >> 4) * 16;
   const uint32_t ba = smem_addr(db) + (n0 + (lane & 7)) * RS + ((lane >> 3) & 1) * 16;
   for (int ks = ks0; ks < steps; ks += TILE == 16 ? 2 : 1) {
-    uint32_t b[NS][2];
+    uint32_t b[NS][2], ma[4];
 #pragma unroll
     for (int s = 0; s < NS; ++s) ldsm2(b[s], ba + s * PL + ks * 32);
 #pragma unroll
@@ -279,10 +294,13 @@ __device__ __forceinline__ void chunk_products(const unsigned char* da, const un
       ldsm4(a, aa + i * PL + ks * 32);
 #pragma unroll
       for (int s = 0; s + i < NS; ++s) mma_f16(acc[i + s], a, b[s][0], b[s][1]);
-      if (i == 0) {
+      if (i == 0)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) a[q] &= 0x7fff7fffu;
-        mma_f16(mag, a, b[0][0] & 0x7fff7fffu, b[0][1] & 0x7fff7fffu);
+        for (int q = 0; q < 4; ++q) ma[q] = a[q];
+      if (i == 1) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) ma[q] = magnitude(ma[q], a[q]);
+        mma_f16(mag, ma, magnitude(b[0][0], b[1][0]), magnitude(b[0][1], b[1][1]));
       }
     }
   }
@@ -307,24 +325,40 @@ __device__ __forceinline__ void chunk_products(const unsigned char* da, const un
     bad[q] = mag[q] < kTrusted && sa != 0 && sb != 0 && m < mt && n < nt;
     nbad += __popc(__ballot_sync(0xffffffffu, bad[q]));
   }
-  // outputs that the digits do not hold well enough, one by one or all at once, whichever is shorter (some 1,000
-  // cycles each, or 400 for every k)
-  if (5 * nbad > 2 * num_k<TILE>(ch.len, ks0)) {
-    plain_products<TILE>(ch, mt, nt, m0, n0, ks0, lane, facc);
-    return;
+  // outputs that the digits do not hold well enough: all at once (256 cycles of the FP64 pipe for every k), or
+  // four at a time (eight for every k and 200)
+  if (nbad > 0) {
+    const int nk = num_k<TILE>(ch.len, ks0);
+    if (nbad * (8 * nk + 200) > 1024 * nk) {
+      plain_products<TILE>(ch, mt, nt, m0, n0, ks0, lane, facc);
+      return;
+    }
+    int at = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t all = __ballot_sync(0xffffffffu, bad[q]);
+      if (bad[q]) list[at + __popc(all & ((1u << lane) - 1))] = (unsigned char)(4 * lane + q);
+      at += __popc(all);
+    }
+    __syncwarp();
+    for (int r = 0; r < nbad; r += 4) {
+      const int id = list[min(r + (lane >> 3), nbad - 1)], l = id >> 2;
+      const int m = m0 + (l >> 2) + (id & 2 ? 8 : 0), n = n0 + 2 * (l & 3) + (id & 1);
+      const double s = ch.alpha == 1.0 ? plain_output<TILE, false>(ch, m, n, ks0, lane & 7)
+                                       : plain_output<TILE, true>(ch, m, n, ks0, lane & 7);
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        const int to = __shfl_sync(0xffffffffu, id, 8 * g);
+        const double x = __shfl_sync(0xffffffffu, s, 8 * g);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (to == 4 * lane + q) w[q] = x;
+      }
+    }
+    __syncwarp();
   }
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    if (!bad[q]) facc[q] = fma(ch.alpha, w[q], facc[q]);
-    if (nbad > 0)
-      for (uint32_t todo = __ballot_sync(0xffffffffu, bad[q]); todo; todo &= todo - 1) {
-        const int l = __ffs(todo) - 1;
-        const double* a = ch.a + (int64_t)(m0 + (l >> 2) + (q & 2 ? 8 : 0)) * ch.asr;
-        const double* b = ch.b + (int64_t)(n0 + 2 * (l & 3) + (q & 1)) * ch.bsr;
-        const double x = plain_output<TILE>(a, ch.ask, b, ch.bsk, ch.len, ch.alpha, ks0, lane);
-        if (lane == l) facc[q] += x;
-      }
-  }
+  for (int q = 0; q < 4; ++q) facc[q] = fma(bad[q] ? 1.0 : ch.alpha, w[q], facc[q]);
 }
 
 template <int KI, int TILE>
@@ -337,6 +371,7 @@ grouped_gemm_f64_kernel(const Tile* __restrict__ tiles, const Term* __restrict__
   __shared__ int ex[2 * TILE];
   __shared__ int flags[2];  // of an even and an odd chunk
   __shared__ int last;
+  __shared__ unsigned char lists[TILE / 4][128];  // outputs of a warp that plain FP64 has to compute
   imps::allow_successor();
   const imps_dslots& slots = planes.s[blockIdx.y];
   if (threadIdx.x == 0) flags[0] = flags[1] = 0;
@@ -387,7 +422,8 @@ grouped_gemm_f64_kernel(const Tile* __restrict__ tiles, const Term* __restrict__
         if (direct)
           plain_products<TILE>(prev, tl.mt, tl.nt, m0, n0, ks0, lane, facc);
         else
-          chunk_products<KI, TILE>(digits, digits + NS * PL, ex, ex + TILE, prev, tl.mt, tl.nt, m0, n0, ks0, lane, facc);
+          chunk_products<KI, TILE>(digits, digits + NS * PL, ex, ex + TILE, lists[warp], prev, tl.mt, tl.nt, m0, n0,
+                                   ks0, lane, facc);
       }
       if (it == tl.nch) break;
       __syncthreads();  // the previous chunk's digits are no longer read

@@ -215,8 +215,9 @@ __global__ void __launch_bounds__(CT) cgs_pass_kernel(const double* __restrict__
 // Block b owns rows [b*sub, (b+1)*sub) of w (sub <= COOP_SUB), kept in shared memory through the
 // three passes; the rows of V that the second pass reads for its dot products are still in L1 when the
 // third reads them for the update.  Each reduction (grid_sums) is one or two grid barriers around sums
-// of the blocks' per-column partials in a fixed order: identical, reproducible results in every block.  Barrier waits are bounded: on timeout *err is
-// set, the remaining work is skipped, and the exit protocol still resets the counters.
+// of the blocks' per-column partials in a fixed order: identical, reproducible results in every block.
+// Barrier waits are bounded: on timeout *err is set, the remaining work is skipped, and the exit
+// protocol still resets the counters.
 // Bound by the FP64 pipe (a warp's FP64 instruction takes 64 cycles of its scheduler whatever its
 // lanes do), so sums over lanes exchange instead of repeat: a warp adds four columns' lane sums with
 // six additions instead of twenty, and the work is laid out so that the four schedulers get equal
@@ -544,13 +545,12 @@ __global__ void gemv_kernel(const double* __restrict__ V, int64_t ldv, int ncols
   }
 }
 
-// y = x / *nrm  (guarded: a zero norm writes zeros and raises the breakdown flag)
 // The tables of one block out (n x kk) = V (n x m) W (m x kk) for the grouped GEMM: slots 2, 0, 1, 32 x 32 tiles,
 // one term.  A thick restart's rotation is a contraction, so it belongs there (split FP16 digits on the tensor
 // cores) and not on the FP64 pipe, whose bound a kernel of its own reached: 48,066 x 126 by 63 columns 1,010
 // -> 113 us, by 1 column 256 -> 47; 2,000 x 32 by 16 38 -> 8; 150,276 x 126 by 63 2,015 -> 338.
-__global__ void rotate_tables_kernel(imps::Term* term, imps::Tile* tiles, int rows, int cols, int n, int ldv, int ldo, int m, int kk,
-                                     int kc) {
+__global__ void rotate_tables_kernel(imps::Term* term, imps::Tile* tiles, int rows, int cols, int n, int ldv,
+                                     int ldo, int m, int kk, int kc) {
   const int id = blockIdx.x * blockDim.x + threadIdx.x;
   if (id == 0) {
     imps::Term t{};
@@ -577,6 +577,7 @@ __global__ void rotate_tables_kernel(imps::Term* term, imps::Tile* tiles, int ro
   tiles[id] = t;
 }
 
+// y = x / *nrm  (guarded: a zero norm writes zeros and raises the breakdown flag)
 __global__ void scale_inv_kernel(const double* __restrict__ x, const double* __restrict__ nrm,
                                  double* __restrict__ y, int64_t n, int* __restrict__ flag, int64_t sx = 0,
                                  int64_t sn = 0, int64_t sy = 0) {
@@ -811,8 +812,8 @@ int kr_basis_rotate(const double* V, int64_t ldv, int m, const double* W, int kk
   const int rows = (int)((n + 31) / 32), cols = (kk + 31) / 32, kc = chunk_len(m);
   Tile* tiles = (Tile*)((char*)scratch + 64);
   imps::count_launch();
-  rotate_tables_kernel<<<(rows * cols + 255) / 256, 256, 0, st>>>((Term*)scratch, tiles, rows, cols, (int)n, (int)ldv, (int)ldo, m,
-                                                                  kk, kc);
+  rotate_tables_kernel<<<(rows * cols + 255) / 256, 256, 0, st>>>((Term*)scratch, tiles, rows, cols, (int)n,
+                                                                  (int)ldv, (int)ldo, m, kk, kc);
   if (cudaGetLastError() != cudaSuccess) return IMPS_ERR_CUDA;
   imps_planes pl{};
   pl.n = 1;
@@ -912,7 +913,8 @@ int kr_axpby(double a, const double* x, double b, double* y, int64_t n, cudaStre
 int kr_proj_epilogue(const double* x, const double* t, const double* s, const double* rho, double* y,
                      int64_t n, cudaStream_t st) {
   imps::count_launch();
-  const cudaError_t e = imps::launch_overlapped(proj_epilogue_kernel, dim3(grid_for(n)), dim3(256), 0, st, x, t, s, rho, y, n);
+  const cudaError_t e =
+      imps::launch_overlapped(proj_epilogue_kernel, dim3(grid_for(n)), dim3(256), 0, st, x, t, s, rho, y, n);
   return e == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
 }
 
@@ -920,14 +922,14 @@ int kr_trace_prod(const KrylovWs& ws, const double* X, const double* R, const in
                   const int32_t* bdim, int nb, double* out, cudaStream_t st, const int32_t* bcols) {
   imps::count_launch();
   constexpr int grid = 128;  // <= RB: the finishing CTA sums the partials of every CTA
-  const cudaError_t e = imps::launch_overlapped(trace_prod_kernel, dim3(grid), dim3(RB), 0, st, X, R, boff, bdim, bcols, nb,
-                                                ws.partials, ws.counter, out);
+  const cudaError_t e = imps::launch_overlapped(trace_prod_kernel, dim3(grid), dim3(RB), 0, st, X, R, boff, bdim,
+                                                bcols, nb, ws.partials, ws.counter, out);
   return e == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
 }
 
 // n doubles and the flags f0, f1 (may be null) to pinned host memory
-__global__ void __launch_bounds__(256) export_kernel(const double* src, int n, const int* f0, const int* f1, double* dst,
-                                                     int* dst_flags) {
+__global__ void __launch_bounds__(256) export_kernel(const double* src, int n, const int* f0, const int* f1,
+                                                     double* dst, int* dst_flags) {
   imps::allow_successor();
   imps::wait_for_predecessor();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -938,8 +940,8 @@ __global__ void __launch_bounds__(256) export_kernel(const double* src, int n, c
 
 int kr_export(const double* src, int n, const int* f0, const int* f1, double* dst, int* dst_flags, cudaStream_t st) {
   imps::count_launch();
-  const cudaError_t e = imps::launch_overlapped(export_kernel, dim3(std::max(1, (n + 255) / 256)), dim3(256), 0, st, src, n,
-                                                f0, f1, dst, dst_flags);
+  const cudaError_t e = imps::launch_overlapped(export_kernel, dim3(std::max(1, (n + 255) / 256)), dim3(256), 0, st,
+                                                src, n, f0, f1, dst, dst_flags);
   return e == cudaSuccess ? IMPS_OK : IMPS_ERR_CUDA;
 }
 

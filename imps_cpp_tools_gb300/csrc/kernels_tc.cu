@@ -183,8 +183,8 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
 // FP64 pipe, slow on this GPU, sees one conversion per element, its bound.  Hubbard D = 1024 H_AC: 17.7
 // us a launch on average with one element per thread, its index divided by rpad and three scattered
 // 2-byte stores; 10.0 now.
-__global__ void __launch_bounds__(256) pack_kernel(const PackJob* __restrict__ jobs, const __grid_constant__ imps_dslots slots,
-                                                   __nv_bfloat16* out) {
+__global__ void __launch_bounds__(256) pack_kernel(const PackJob* __restrict__ jobs,
+                                                   const __grid_constant__ imps_dslots slots, __nv_bfloat16* out) {
   imps::allow_successor();
   const PackJob jb = jobs[blockIdx.x];
   const double* S = slots.p[jb.slot] + jb.src_off;
@@ -203,7 +203,9 @@ __global__ void __launch_bounds__(256) pack_kernel(const PackJob* __restrict__ j
     float xf[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e)
-      xf[e] = r < jb.rows && k0 + e < jb.k ? __double2float_rn(S[(int64_t)(jb.r0 + r) * sr + (int64_t)(k0 + e) * sk]) * alpha : 0.0f;
+      xf[e] = r < jb.rows && k0 + e < jb.k
+                  ? __double2float_rn(S[(int64_t)(jb.r0 + r) * sr + (int64_t)(k0 + e) * sk]) * alpha
+                  : 0.0f;
     __nv_bfloat162 w[3][4];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
@@ -227,7 +229,8 @@ __global__ void __launch_bounds__(256) pack_kernel(const PackJob* __restrict__ j
 // warp
 __device__ __forceinline__ double widen(float x) {
   const uint32_t b = __float_as_uint(x), mag = b & 0x7fffffffu;
-  if (mag - 0x00800000u < 0x7f000000u) return __hiloint2double((int)((b & 0x80000000u) | ((mag >> 3) + 0x38000000u)), (int)(b << 29));
+  if (mag - 0x00800000u < 0x7f000000u)
+    return __hiloint2double((int)((b & 0x80000000u) | ((mag >> 3) + 0x38000000u)), (int)(b << 29));
   return mag == 0 ? __hiloint2double((int)b, 0) : (double)x;
 }
 
@@ -482,7 +485,8 @@ int tc_create(TcPlan** out, const Plan& P, cudaStream_t st) {
       for (int e = t.t0; e < t.t1; ++e) k += ts.terms[e].ksteps;
       return k * t.npad;
     };
-    std::stable_sort(ts.tiles.begin(), ts.tiles.end(), [&](const TcTile& a, const TcTile& b) { return work(a) > work(b); });
+    std::stable_sort(ts.tiles.begin(), ts.tiles.end(),
+                     [&](const TcTile& a, const TcTile& b) { return work(a) > work(b); });
     T->stages.push_back(std::move(ts));
   }
   T->packed_elems = off;
