@@ -38,9 +38,9 @@
 // mma.sync rather than tcgen05: the operands are split in registers on the fly (no operand packs that
 // could go stale, no extra pass over memory), blocks are ragged with edges from 1 to 82, and the eight
 // level sums of a 16 x 8 sub-tile fit a warp's registers, where a 128-row instruction would compute
-// mostly padding.  What bounds it (XXZ D = 512 H_AC, ncu): integer pipe 29%, tensor pipe 16%, FP64 pipe
-// 13% busy, i.e. the latency of the chain load - split - multiply - combine of one to three chunks per
-// CTA; throughput alone would take about 5 us.
+// mostly padding.  What bounds it (XXZ D = 512 H_AC, ncu): integer pipe 28%, tensor pipe 19%, FP64 pipe
+// 12% busy, i.e. the latency of the chain load - split - multiply - combine of one to three chunks per
+// CTA; throughput alone would take about 6 us.
 //
 // Work split: a table entry is an output tile (<= 32 x 32, or <= 16 x 16 where a stage has too few
 // tiles; edges are multiples of 16 and 8, balanced over the block, so that a 68 x 68 block computes

@@ -548,7 +548,8 @@ __global__ void gemv_kernel(const double* __restrict__ V, int64_t ldv, int ncols
 // The tables of one block out (n x kk) = V (n x m) W (m x kk) for the grouped GEMM: slots 2, 0, 1, 32 x 32 tiles,
 // one term.  A thick restart's rotation is a contraction, so it belongs there (split FP16 digits on the tensor
 // cores) and not on the FP64 pipe, whose bound a kernel of its own reached: 48,066 x 126 by 63 columns 1,010
-// -> 113 us, by 1 column 256 -> 47; 2,000 x 32 by 16 38 -> 8; 150,276 x 126 by 63 2,015 -> 338.
+// -> 132 us (294 in a VUMPS sweep, where the first column's outputs mostly go to plain FP64; 847 before), by 1
+// column 256 -> 55; 2,000 x 32 by 16 38 -> 10; 150,276 x 126 by 63 2,015 -> 389.
 __global__ void rotate_tables_kernel(imps::Term* term, imps::Tile* tiles, int rows, int cols, int n, int ldv,
                                      int ldo, int m, int kk, int kc) {
   const int id = blockIdx.x * blockDim.x + threadIdx.x;
