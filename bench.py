@@ -53,8 +53,8 @@ APPLIES_PER_STEP = 20
 L2_FLUSH_BYTES = 512 << 20
 # DRAM bytes (read + write) of one H_AC apply from one ncu capture of `bench.py --mode hac`
 # (profiles/tc_gemm_hac_xxz_d512.md: tc_gemm 2.73 MB, and 0.40 MB of the pack's input;
-# profiles/grouped_gemm_f64_hac_xxz_d512.md, autotuned shape 32x32 with 4 shares: 2.39 MB)
-NCU_TRAFFIC_BYTES = {"bf16x6": 3.13e6, "fp64": 2.39e6}
+# profiles/grouped_gemm_f64_hac_xxz_d512.md, autotuned shape 32x32 with 4 shares: 2.40 MB)
+NCU_TRAFFIC_BYTES = {"bf16x6": 3.13e6, "fp64": 2.40e6}
 FP16_DIGIT_PRODUCTS = 37  # 36 of the digits, one of the first digits' magnitudes
 # tolerances of the timed sweeps: the eigensolver tolerance of the configuration (1e-12); GMRES
 # 1e-8, because the environment systems of these states do not reach 1e-12 in floating point:
